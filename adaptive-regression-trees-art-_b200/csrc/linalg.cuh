@@ -371,6 +371,94 @@ __device__ void warp_backward(const T* L, V* z, int p) {
   }
 }
 
+// One warp's Cholesky solve of the augmented system [G h; h^T .] (packed
+// lower, p + 1 rows, p + 1 <= 32 RPL): G = L L^T in place, the last row
+// carried along as one more row of the panel, so that it ends as L^{-1} h and
+// only the back substitution is left; the solution goes to x[0..p).  Returns
+// 0, or the 1-based index of the first pivot that is not positive and finite.
+//
+// Latency-bound: column j is one dot product per lane (rows lane + 32 m, left
+// looking, two partial sums), one reciprocal square root (a double square
+// root and a division in a row cost about 220 cycles, rsqrt 70) and one
+// barrier; the back substitution keeps its vector in registers and passes
+// each unknown by shuffle.
+template <int RPL>
+__device__ int warp_chol_solve(double* A, int p, double* x) {
+  const int lane = threadIdx.x & 31;
+  double inv[RPL];
+  const double* row[RPL];
+#pragma unroll
+  for (int m = 0; m < RPL; ++m) {
+    inv[m] = 0.0;
+    row[m] = A + pk(min(lane + 32 * m, p), 0);
+  }
+  __syncwarp();
+  for (int j = 0; j < p; ++j) {
+    const double* rj = A + pk(j, 0);
+    double t[RPL], u[RPL];
+#pragma unroll
+    for (int m = 0; m < RPL; ++m) {
+      t[m] = lane + 32 * m >= j ? row[m][j] : 0.0;
+      u[m] = 0.0;
+    }
+    int k = 0;
+#pragma unroll 2
+    for (; k + 1 < j; k += 2) {
+      const double w0 = rj[k], w1 = rj[k + 1];
+#pragma unroll
+      for (int m = 0; m < RPL; ++m) {
+        t[m] = fma(-row[m][k], w0, t[m]);
+        u[m] = fma(-row[m][k + 1], w1, u[m]);
+      }
+    }
+    if (k < j) {
+      const double w0 = rj[k];
+#pragma unroll
+      for (int m = 0; m < RPL; ++m) t[m] = fma(-row[m][k], w0, t[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < RPL; ++m) t[m] += u[m];
+    double dj = __shfl_sync(0xffffffffu, t[0], j & 31);
+#pragma unroll
+    for (int m = 1; m < RPL; ++m) {
+      const double o = __shfl_sync(0xffffffffu, t[m], j & 31);
+      if ((j >> 5) == m) dj = o;
+    }
+    if (!(dj > 0.0) || !isfinite(dj)) return j + 1;
+    const double rs = rsqrt(dj);
+    __syncwarp();  // every lane has read column j
+#pragma unroll
+    for (int m = 0; m < RPL; ++m) {
+      const int i = lane + 32 * m;
+      if (i >= j && i <= p) A[pk(i, j)] = t[m] * rs;
+      if (i == j) inv[m] = rs;
+    }
+    __syncwarp();
+  }
+  double z[RPL];
+#pragma unroll
+  for (int m = 0; m < RPL; ++m) {
+    const int i = lane + 32 * m;
+    z[m] = i < p ? A[pk(p, i)] : 0.0;
+  }
+  for (int j = p - 1; j >= 0; --j) {
+    double xj = __shfl_sync(0xffffffffu, z[0] * inv[0], j & 31);
+#pragma unroll
+    for (int m = 1; m < RPL; ++m) {
+      const double o = __shfl_sync(0xffffffffu, z[m] * inv[m], j & 31);
+      if ((j >> 5) == m) xj = o;
+    }
+#pragma unroll
+    for (int m = 0; m < RPL; ++m) {
+      const int i = lane + 32 * m;
+      if (i < j) z[m] = fma(-A[pk(j, i)], xj, z[m]);
+      else if (i == j) x[j] = xj;
+    }
+  }
+  __syncwarp();
+  return 0;
+}
+
 // 1-norm of the symmetric matrix held in packed lower storage (one warp).
 template <typename T>
 __device__ double warp_sym_norm1(const T* A, int p) {

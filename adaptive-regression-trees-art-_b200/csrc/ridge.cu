@@ -9,13 +9,15 @@
 // art/_cuda_batched_cholesky_kernels.cu:138-148).
 //
 // Launch sequence (all stream-ordered, no host sync):
-//   plan_hist -> plan_scan -> plan_scatter : per-class work lists, largest
+//   plan_hist -> plan_scan -> plan_scatter (plan_small: one launch for up to
+//       2,048 systems)                     : per-class work lists, largest
 //       cost first (log2 buckets of n*(p+1)^2), built on the device;
 //   [mixed] ridge_tc_kernel                : tcgen05 Gram + refinement;
-//   ridge_warp_kernel                      : FP64, (p+1) <= 24, warp per system;
-//   ridge_fp64_kernel<4>, <8>              : persistent FP64 work queues
-//       (<4>: Gram on the FP64 tensor cores, mma.sync m8n8k4; <8>: 8x8
-//       FP64 register tiles);
+//   ridge_dmma_kernel<6>, <3>              : FP64, (p+1) <= 48, warps alone on
+//       FP64 MMA Grams (ridge_dmma.cu); ridge_split_finish for the systems
+//       it split over several warps;
+//   ridge_fp64_kernel<8>                   : FP64, wider systems, persistent
+//       queue, 8x8 register tiles;
 //   ridge_fp64_kernel<8> on the resolve list (mixed systems that did not
 //       converge); ridge_qr_kernel on the auto-solver fallback list.
 #include <stdarg.h>
@@ -46,60 +48,160 @@ __device__ __forceinline__ int plan_bucket(int64_t n, int p) {
   return kBuckets - 1 - max(0, min(kBuckets - 1, e));  // bucket 0 = largest
 }
 
-// Validate each item, pick its class and cost bucket, count.
+// The split classes' cost of n rows: MMAs a row tile plus what forming it takes.
+__device__ __forceinline__ unsigned long long split_cost(int64_t n, int pa) {
+  const int nb = (pa + 7) / 8;
+  return (unsigned long long)n * (unsigned)(nb * (nb + 1) / 2 + 3);
+}
+__device__ __forceinline__ int split_class(int c) { return c == CLS_WARP ? 0 : (c == CLS_SMALL ? 1 : -1); }
+
+// Validate item k, pick its class and cost bucket; -1: no kernel takes it
+// (`report`: its status is written).
+__device__ __forceinline__ int plan_item(const RidgeArgs& a, int64_t k, bool report, int64_t& n, int& p) {
+  const int d = a.dims[k], kind = a.features[k];
+  p = feature_count(d, kind);
+  n = a.row_offsets[k + 1] - a.row_offsets[k];
+  if (d < 1 || d > a.dmax || p < 1 || p > a.pmax || n < 0) {
+    if (report) {
+      const double nan = __longlong_as_double(0x7ff8000000000000ll);
+      a.status[k] = -4;
+      if (a.ridge_eff) a.ridge_eff[k] = nan;
+      if (a.cond) a.cond[k] = nan;
+      if (a.info) a.info[k] = 0u;
+      for (int i = 0; i < a.pmax; ++i) a.beta[k * a.beta_stride + i] = nan;
+    }
+    return -1;
+  }
+  const int c = plan_class(a, p);
+  if (c < 0 && report) a.status[k] = -4;
+  return c;
+}
+
+// Place item k: on its class's list at `slot`, or, when it costs more than a
+// warp's share of its class and the pool has room, as a split system (a run
+// of units per queue entry, about a quarter of a share each).  `slot` is the
+// list position it would take; a split item leaves its place to a zero-cost
+// marker (-1).
+__device__ void plan_place(const RidgeArgs& a, const RidgeLists& L, int64_t k, int c, int slot, int64_t n, int p) {
+  const int sc = split_class(c);
+  int32_t entry = (int32_t)k;
+  if (sc >= 0 && L.pool_cap > 0) {
+    const int pa = p + 1, E = pa * (pa + 1) / 2;
+    const int64_t U = ridge_unit_rows(n);
+    const int nseg = (int)((n + U - 1) / U);
+    const unsigned long long share = __ldcg(&L.cost[sc]) / (unsigned)max(L.workers[sc], 1);
+    if (nseg > 1 && split_cost(n, pa) > share) {
+      const unsigned long long need = (unsigned long long)nseg * E;
+      const unsigned long long at = atomicAdd(L.pool_used, need);
+      if (at + need <= (unsigned long long)L.pool_cap) {
+        const int r = atomicAdd(L.nrec, 1);
+        if (r < L.rec_cap) {
+          const int run = (int)max(1ull, min(share / (4 * split_cost(U, pa)), (unsigned long long)nseg));
+          const int m = (nseg + run - 1) / run;
+          const int i0 = atomicAdd(&L.nitems[sc], m);
+          const bool fits = i0 + m <= L.item_cap;
+          for (int j = 0; j < m && i0 + j < L.item_cap; ++j)
+            L.items[(int64_t)sc * L.item_cap + i0 + j] = fits ? make_int4(r, j * run, run, 0) : make_int4(-1, 0, 0, 0);
+          SplitRec rec;
+          rec.base = (int64_t)at;
+          rec.k = fits ? (int32_t)k : -1;
+          rec.nseg = nseg;
+          rec.bad = 0;
+          rec.pad = 0;
+          L.recs[r] = rec;
+          if (fits) entry = -1;
+        }
+      }
+    }
+  }
+  L.list[(int64_t)c * a.K + slot] = entry;
+}
+
+// Count each class's items by cost bucket.
 __global__ void ridge_plan_hist(RidgeArgs a, RidgeLists L) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.K) return;
-  const int d = a.dims[k], kind = a.features[k];
-  const int p = feature_count(d, kind);
-  const int64_t n = a.row_offsets[k + 1] - a.row_offsets[k];
-  if (d < 1 || d > a.dmax || p < 1 || p > a.pmax || n < 0) {
-    const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    a.status[k] = -4;
-    if (a.ridge_eff) a.ridge_eff[k] = nan;
-    if (a.cond) a.cond[k] = nan;
-    if (a.info) a.info[k] = 0u;
-    for (int i = 0; i < a.pmax; ++i) a.beta[k * a.beta_stride + i] = nan;
-    return;
-  }
-  const int c = plan_class(a, p);
-  if (c < 0) {
-    a.status[k] = -4;
-    return;
-  }
+  int64_t n;
+  int p;
+  const int c = plan_item(a, k, true, n, p);
+  if (c < 0) return;
   atomicAdd(&L.hist[c * kBuckets + plan_bucket(n, p)], 1);
+  if (split_class(c) >= 0) atomicAdd(&L.cost[split_class(c)], split_cost(n, p + 1));
 }
 
-__global__ void ridge_plan_scan(RidgeLists L) {
-  // one block of kPlanClasses warps; warp c scans class c's buckets
-  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (c >= kPlanClasses) return;
+__device__ __forceinline__ void plan_scan_class(const int* hist, int* start, int32_t* count, int c) {
+  const int lane = threadIdx.x & 31;
   int carry = 0;
   for (int base = 0; base < kBuckets; base += 32) {
-    int v = L.hist[c * kBuckets + base + lane];
+    int v = hist[c * kBuckets + base + lane];
     int incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       int t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
-    L.start[c * kBuckets + base + lane] = carry + incl - v;
+    start[c * kBuckets + base + lane] = carry + incl - v;
     carry += __shfl_sync(0xffffffffu, incl, 31);
   }
-  if (lane == 0) L.count[c] = carry;
+  if (lane == 0) count[c] = carry;
+}
+
+__global__ void ridge_plan_scan(RidgeLists L) {
+  // one block of kPlanClasses warps; warp c scans class c's buckets
+  const int c = threadIdx.x >> 5;
+  if (c < kPlanClasses) plan_scan_class(L.hist, L.start, L.count, c);
 }
 
 __global__ void ridge_plan_scatter(RidgeArgs a, RidgeLists L) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.K) return;
-  const int d = a.dims[k], kind = a.features[k];
-  const int p = feature_count(d, kind);
-  const int64_t n = a.row_offsets[k + 1] - a.row_offsets[k];
-  if (d < 1 || d > a.dmax || p < 1 || p > a.pmax || n < 0) return;
-  const int c = plan_class(a, p), b = plan_bucket(n, p);
+  int64_t n;
+  int p;
+  const int c = plan_item(a, k, false, n, p);
   if (c < 0) return;
+  const int b = plan_bucket(n, p);
   const int slot = atomicSub(&L.hist[c * kBuckets + b], 1) - 1;
-  L.list[(int64_t)c * a.K + L.start[c * kBuckets + b] + slot] = (int32_t)k;
+  plan_place(a, L, k, c, L.start[c * kBuckets + b] + slot, n, p);
+}
+
+// The whole plan of a small batch in one CTA: the header cleared, histogram,
+// scan and placement with block barriers between them (one launch in place of
+// a memset and three; 5 us against 12 us for one system).
+constexpr int kPlanOneCta = 2048;
+__device__ __forceinline__ int plan_level(int64_t n) { return ilogb((double)ridge_unit_rows(n)) - 8; }
+__global__ void __launch_bounds__(1024) ridge_plan_small(RidgeArgs a, RidgeLists L, int32_t* header, int header_words) {
+  __shared__ int hist[kPlanClasses * kBuckets], start[kPlanClasses * kBuckets], s_level;
+  if (threadIdx.x == 0) s_level = 0;
+  for (int i = threadIdx.x; i < header_words; i += 1024) header[i] = 0;
+  for (int i = threadIdx.x; i < kPlanClasses * kBuckets; i += 1024) hist[i] = 0;
+  __threadfence();
+  __syncthreads();
+  for (int64_t k = threadIdx.x; k < a.K; k += 1024) {
+    int64_t n;
+    int p;
+    const int c = plan_item(a, k, true, n, p);
+    if (c < 0) continue;
+    atomicAdd(&hist[c * kBuckets + plan_bucket(n, p)], 1);
+    atomicMax(&s_level, plan_level(n));
+    if (split_class(c) >= 0) atomicAdd(&L.cost[split_class(c)], split_cost(n, p + 1));
+  }
+  __threadfence();
+  __syncthreads();
+  if ((threadIdx.x >> 5) < kPlanClasses) plan_scan_class(hist, start, L.count, threadIdx.x >> 5);
+  __syncthreads();
+  // longest units first, so that the queue ends with the short ones and the
+  // pool, should it run out, runs out for the small systems
+  for (int level = s_level; level >= 0; --level) {
+    for (int64_t k = threadIdx.x; k < a.K; k += 1024) {
+      int64_t n;
+      int p;
+      const int c = plan_item(a, k, false, n, p);
+      if (c < 0 || plan_level(n) != level) continue;
+      const int b = plan_bucket(n, p);
+      plan_place(a, L, k, c, start[c * kBuckets + b] + atomicSub(&hist[c * kBuckets + b], 1) - 1, n, p);
+    }
+    __syncthreads();
+  }
 }
 
 // ============================================================ FP64 kernel
@@ -119,28 +221,10 @@ __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~(size_t
 __host__ __device__ inline int phi_pos(int ts, int blk, int j) { return blk * ts + ((j + blk) & (ts - 1)); }
 __host__ __device__ inline int phi_stride(int ts, int nb) { return nb * ts; }
 
-// Row stride of the phi tile in the 4-feature-block kernel, which forms the
-// Gram with FP64 tensor-core MMAs (m8n8k4): 8-feature blocks, stride = 8
-// (mod 16) doubles so that a fragment load (4 rows x 8 features) touches
-// every bank pair exactly twice.
-__host__ __device__ inline int dmma_stride(int pa) {
-  const int nb8 = (pa + 7) / 8;
-  return 8 * nb8 + ((nb8 & 1) ? 0 : 8);
-}
-
-// D (8x8, two doubles per lane) += A (8x4) * B (4x8) in FP64 on the tensor
-// cores.  Lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4) + {0,1}].
-__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
 __host__ __device__ inline Fp64Layout fp64_layout(int pmax, int dmax, int ts, int chunk) {
   Fp64Layout L;
   const int pa = pmax + 1;
-  // features incl. padding: 8-feature blocks in the tensor-core form (ts = 4)
-  L.ldp = ts == 4 ? ((pa + 7) / 8) * 8 : ((pa + ts - 1) / ts) * ts;
+  L.ldp = ((pa + ts - 1) / ts) * ts;  // features incl. padding
   L.chunk = chunk;
   size_t o = 0;
   for (int s = 0; s < 2; ++s) {
@@ -150,7 +234,7 @@ __host__ __device__ inline Fp64Layout fp64_layout(int pmax, int dmax, int ts, in
   }
   L.off_bar = o; o = align16(o + 2 * 8);
   L.off_phi = o;
-  o = align16(o + (size_t)chunk * (ts == 4 ? dmma_stride(pa) : phi_stride(ts, L.ldp / ts)) * 8);
+  o = align16(o + (size_t)chunk * phi_stride(ts, L.ldp / ts) * 8);
   L.off_q = o; o = align16(o + (size_t)chunk * 8);
   L.off_gram = o; o = align16(o + (size_t)pa * (pa + 1) / 2 * 8);
   L.off_fa = o; o = align16(o + (size_t)L.ldp * 2);
@@ -175,9 +259,8 @@ __device__ __forceinline__ void issue_chunk(const RidgeArgs& a, const RidgeItem&
   if (a.w) bulk_g2s(smem + lay.off_w[st], gw.base, gw.bytes, bar);
 }
 
-// TS = 4 (tensor-core Gram, 80 registers) is held to three CTAs per SM.
 template <int TS, int CHUNK>
-__global__ void __launch_bounds__(kRidgeThreads, TS == 4 ? 3 : 1) ridge_fp64_kernel(RidgeArgs a, RidgeLists L,
+__global__ void __launch_bounds__(kRidgeThreads, 1) ridge_fp64_kernel(RidgeArgs a, RidgeLists L,
                                                                    int cls, int pcap) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_item, s_fail;
@@ -208,13 +291,11 @@ __global__ void __launch_bounds__(kRidgeThreads, TS == 4 ? 3 : 1) ridge_fp64_ker
     const int k = L.list[(int64_t)cls * a.K + item];
     const RidgeItem it = load_item(a, k);
     const int p = it.p, pa = p + 1, d = it.d;
-    // TS = 4: FP64 tensor-core tiles of 8 features; TS = 8: 8x8 register tiles
-    constexpr bool kDmma = TS == 4;
-    const int nb = kDmma ? (pa + 7) / 8 : (pa + TS - 1) / TS;
-    const int ldpi = kDmma ? 8 * nb : nb * TS;            // features incl. padding
-    const int lds = kDmma ? dmma_stride(pa) : phi_stride(TS, nb);  // phi row stride
+    const int nb = (pa + TS - 1) / TS;
+    const int ldpi = nb * TS;             // features incl. padding
+    const int lds = phi_stride(TS, nb);   // phi row stride
     const int T = nb * (nb + 1) / 2;
-    const int S = kDmma ? 1 : max(1, kRidgeThreads / T);
+    const int S = max(1, kRidgeThreads / T);
     for (int f = tid; f < ldpi; f += kRidgeThreads) {
       int fa_, fb_;
       if (f < p) feature_factors(d, it.kind, f, fa_, fb_);
@@ -231,16 +312,6 @@ __global__ void __launch_bounds__(kRidgeThreads, TS == 4 ? 3 : 1) ridge_fp64_ker
     for (int i = 0; i < TS; ++i)
 #pragma unroll
       for (int j = 0; j < TS; ++j) acc[i][j] = 0.0;
-    // tensor-core form: warp w owns 8x8 tiles w, w + 8, w + 16 (T <= 21)
-    const int wid = tid >> 5, wl = tid & 31;
-    double dacc[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-    int tI[3], tJ[3];
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      const int t2 = wid + 8 * m;
-      tI[m] = t2 < T ? tile_row(t2) : 0;
-      tJ[m] = t2 < T ? t2 - tI[m] * (tI[m] + 1) / 2 : 0;
-    }
     int bad = 0;
     const int64_t nchunks = (it.n + CHUNK - 1) / CHUNK;
     if (tid == 0) {
@@ -277,37 +348,22 @@ __global__ void __launch_bounds__(kRidgeThreads, TS == 4 ? 3 : 1) ridge_fp64_ker
       // phi[r][phi_pos(blk, j)] = sqrt(q_r) * feature(blk*TS + j): the
       // rotation and shift spread the tiles' loads over distinct banks.
       const int warp = tid >> 5, lane = tid & 31;
-      // the tensor-core form reads rows in groups of 4: pad with zero rows
-      const int rows_pad = kDmma ? (rows + 3) & ~3 : rows;
-      for (int r = warp; r < rows_pad; r += kRidgeThreads / 32) {
-        const bool live = r < rows;
-        const double* xr = xs + (int64_t)(live ? r : 0) * d;
-        const double sq = live ? q[r] : 0.0;
+      for (int r = warp; r < rows; r += kRidgeThreads / 32) {
+        const double* xr = xs + (int64_t)r * d;
+        const double sq = q[r];
         for (int f = lane; f < ldpi; f += 32) {
           const int ia = fa[f], ib = fb[f];
           double v;
-          if (ia == -3 || !live) v = 0.0;
+          if (ia == -3) v = 0.0;
           else if (ia == -2) v = sq * ys[r];
           else v = sq * ((ia < 0 ? 1.0 : xr[ia]) * (ib < 0 ? 1.0 : xr[ib]));
-          if constexpr (kDmma) {
-            phi[r * lds + f] = v;
-          } else {
-            const int blk = f / TS, j = f - blk * TS;
-            phi[r * lds + phi_pos(TS, blk, j)] = v;
-          }
+          const int blk = f / TS, j = f - blk * TS;
+          phi[r * lds + phi_pos(TS, blk, j)] = v;
         }
       }
       __syncthreads();
       if (tid == 0 && c + 2 < nchunks) issue_chunk(a, it, CHUNK, c + 2, smem, lay, st, &bars[st]);
-      if constexpr (kDmma) {
-        const int off = (wl & 3) * lds + (wl >> 2);
-        for (int k0 = 0; k0 < rows_pad; k0 += 4) {
-          const double* pr = phi + k0 * lds + off;
-#pragma unroll
-          for (int m = 0; m < 3; ++m)
-            if (wid + 8 * m < T) dmma_884(dacc[m], pr[8 * tI[m]], pr[8 * tJ[m]]);
-        }
-      } else if (mine) {
+      if (mine) {
         for (int r = slice; r < rows; r += S) {
           const double* pr = phi + r * lds;
           double av[TS], bv[TS];
@@ -340,21 +396,8 @@ __global__ void __launch_bounds__(kRidgeThreads, TS == 4 ? 3 : 1) ridge_fp64_ker
       const int bw = __syncthreads_or(bad & 2), bx = __syncthreads_or(bad & 1);
       bad = (bw ? 2 : 0) | (bx ? 1 : 0);
     }
-    if constexpr (kDmma) {  // each lower entry belongs to one warp's tile
-#pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        if (wid + 8 * m >= T) continue;
-        const int r = 8 * tI[m] + (wl >> 2);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int cc = 8 * tJ[m] + 2 * (wl & 3) + e;
-          if (r < pa && cc <= r) G[pk(r, cc)] = dacc[m][e];
-        }
-      }
-      __syncthreads();
-    }
     // deterministic slice reduction into the packed augmented Gram
-    for (int s = 0; s < (kDmma ? 0 : S); ++s) {
+    for (int s = 0; s < S; ++s) {
       if (mine && slice == s) {
 #pragma unroll
         for (int i = 0; i < TS; ++i)
@@ -691,13 +734,34 @@ static constexpr WsLayout ws_layout(int64_t K) {
   w.off_cursor = o; o += kClasses * 4;
   w.off_hist = o; o += kPlanClasses * kBuckets * 4;
   w.off_start = o; o += kPlanClasses * kBuckets * 4;
-  w.off_err = o; o += 16;
+  w.off_err = o; o += 64;  // error flag, split records, queue entries, costs, pool cursor
   w.header = o;  // zeroed every call
   o = (o + 255) & ~(size_t)255;
   w.off_lambda = o; o += (size_t)K * 8;
   o = (o + 255) & ~(size_t)255;
   w.off_list = o; o += (size_t)kClasses * K * 4;
   w.total = (o + 255) & ~(size_t)255;
+  return w;
+}
+
+// Split systems' records, queue entries and unit Grams, behind the lists in
+// the workspace.  All optional: with less room fewer systems are split, with
+// the same results.
+struct SplitLayout {
+  size_t off_recs, off_items, off_pool, total;
+  int rec_cap, item_cap;
+};
+static SplitLayout split_layout(int64_t K, int max_features, size_t at) {
+  SplitLayout w{};
+  w.total = at;
+  if (K < 1 || K > kSplitMaxCount) return w;
+  w.rec_cap = (int)std::min<int64_t>(K, kSplitRecs);
+  w.item_cap = (int)std::min<int64_t>(K * kMaxUnits, kSplitItems);
+  const int64_t pa = std::min(max_features, kSmallMaxAug - 1) + 1, per = kMaxUnits * (pa * (pa + 1) / 2);
+  w.off_recs = at;
+  w.off_items = (w.off_recs + (size_t)w.rec_cap * sizeof(SplitRec) + 255) & ~(size_t)255;
+  w.off_pool = (w.off_items + (size_t)2 * w.item_cap * sizeof(int4) + 255) & ~(size_t)255;
+  w.total = w.off_pool + ((std::min<size_t>((size_t)K * per * 8, kSplitPoolBytes) + 255) & ~(size_t)255);
   return w;
 }
 
@@ -730,9 +794,8 @@ static int launch_persistent(Kern kern, size_t smem, int64_t max_items, cudaStre
 using namespace art;
 
 extern "C" size_t art_ridge_workspace_size(int64_t count, int32_t max_features) {
-  (void)max_features;
   if (count < 0) return 0;
-  return ws_layout(count).total;
+  return split_layout(count, std::max(max_features, 1), ws_layout(count).total).total;
 }
 
 static int ridge_entry(const ArtRidgeProblem* pr, const ArtRidgeResult* res, float* gram_out,
@@ -802,7 +865,7 @@ static int ridge_entry(const ArtRidgeProblem* pr, const ArtRidgeResult* res, flo
   a.ridge_eff = res->ridge_effective; a.cond = res->cond_estimate;
   a.status = res->status; a.info = res->info;
   a.options = pr->options;
-  a.tensor_min_p = pr->tensor_min_features > 0 ? std::max(pr->tensor_min_features, kTensorMinP) : kTensorMinP;
+  a.tensor_min_p = pr->tensor_min_features > 0 ? std::max(pr->tensor_min_features, kTensorMinP) : kTensorDefaultP;
   if (gram_out) a.tensor_min_p = kTensorMinP;
   a.gram_out = gram_out;
   a.gram_stride = gram_stride;
@@ -815,38 +878,67 @@ static int ridge_entry(const ArtRidgeProblem* pr, const ArtRidgeResult* res, flo
   L.err = (int32_t*)(ws + wl.off_err);
   L.lambda = (double*)(ws + wl.off_lambda);
   L.list = (int32_t*)(ws + wl.off_list);
-  if (cudaMemsetAsync(ws, 0, wl.header, s) != cudaSuccess) return check_launch("memset");
-  const unsigned pg = (unsigned)((K + 255) / 256);
+  L.nrec = L.err + 1;
+  L.nitems = L.err + 2;
+  L.cost = (unsigned long long*)(L.err + 4);
+  L.pool_used = L.cost + 2;
+  const SplitLayout sl = split_layout(K, a.pmax, wl.total);
+  L.recs = (SplitRec*)(ws + sl.off_recs);
+  L.items = (int4*)(ws + sl.off_items);
+  L.pool = (double*)(ws + sl.off_pool);
+  L.pool_cap = sl.total > wl.total && ws_bytes > sl.off_pool
+                   ? (int64_t)((std::min(ws_bytes, sl.total) - sl.off_pool) / sizeof(double)) : 0;
+  if (gram_out) L.pool_cap = 0;
+  L.rec_cap = L.pool_cap > 0 ? sl.rec_cap : 0;
+  L.item_cap = L.pool_cap > 0 ? sl.item_cap : 0;
+  const bool has_small = a.pmax + 1 > kWarpMaxAug;
+  if (!gram_out) {
+    L.workers[0] = 4 * ridge_dmma_ctas(CLS_WARP);
+    L.workers[1] = has_small ? 4 * ridge_dmma_ctas(CLS_SMALL) : 0;
+    if (L.workers[0] < 1 || (has_small && L.workers[1] < 1)) {
+      set_error("art_ridge_batched: cannot reserve shared memory for the FP64 kernels");
+      return ART_E_UNSUPPORTED;
+    }
+  }
   prof_begin("ridge_plan", s);
-  ridge_plan_hist<<<pg, 256, 0, s>>>(a, L);
-  ridge_plan_scan<<<1, 32 * kPlanClasses, 0, s>>>(L);
-  ridge_plan_scatter<<<pg, 256, 0, s>>>(a, L);
+  if (K <= kPlanOneCta) {
+    ridge_plan_small<<<1, 1024, 0, s>>>(a, L, (int32_t*)ws, (int)(wl.header / 4));
+    count_launch();
+  } else {
+    if (cudaMemsetAsync(ws, 0, wl.header, s) != cudaSuccess) return check_launch("memset");
+    const unsigned pg = (unsigned)((K + 255) / 256);
+    ridge_plan_hist<<<pg, 256, 0, s>>>(a, L);
+    ridge_plan_scan<<<1, 32 * kPlanClasses, 0, s>>>(L);
+    ridge_plan_scatter<<<pg, 256, 0, s>>>(a, L);
+    count_launch();
+    count_launch();
+    count_launch();
+  }
   prof_end(s);
-  count_launch();
-  count_launch();
-  count_launch();
   int rc = check_launch("ridge plan");
   if (rc) return rc;
-  if (a.precision == ART_PRECISION_MIXED) {
+  if (a.precision == ART_PRECISION_MIXED && (gram_out || a.pmax >= a.tensor_min_p)) {
     rc = launch_ridge_tensor(a, L, s);
     if (rc) return rc;
   }
   if (gram_out) return ART_OK;
-  rc = launch_ridge_warp(a, L, s);
-  if (rc) return rc;
-  if (a.pmax + 1 > kWarpMaxAug) {
-    const int pcap = std::min(a.pmax, kSmallMaxAug - 1);
-    const size_t sm = fp64_layout(pcap, a.dmax, 4, 64).total;
-    rc = launch_persistent(ridge_fp64_kernel<4, 64>, sm, K, s, a, L, CLS_SMALL, pcap,
-                           "ridge_fp64<4>");
+  if (has_small) {
+    rc = launch_ridge_dmma(a, L, CLS_SMALL, s);
     if (rc) return rc;
   }
-  if (a.pmax + 1 > kSmallMaxAug || a.precision == ART_PRECISION_MIXED) {
+  rc = launch_ridge_dmma(a, L, CLS_WARP, s);
+  if (rc) return rc;
+  if (L.pool_cap > 0) {
+    rc = launch_ridge_split_finish(a, L, s);
+    if (rc) return rc;
+  }
+  const bool tensor = a.precision == ART_PRECISION_MIXED && a.pmax >= a.tensor_min_p;
+  if (a.pmax + 1 > kSmallMaxAug || tensor) {
     const size_t sm = fp64_layout(a.pmax, a.dmax, 8, 32).total;
     rc = launch_persistent(ridge_fp64_kernel<8, 32>, sm, K, s, a, L, CLS_LARGE, a.pmax,
                            "ridge_fp64<8>");
     if (rc) return rc;
-    if (a.precision == ART_PRECISION_MIXED) {
+    if (tensor) {
       rc = launch_persistent(ridge_fp64_kernel<8, 32>, sm, K, s, a, L, CLS_RESOLVE, a.pmax,
                              "ridge_fp64<8> resolve");
       if (rc) return rc;

@@ -12,10 +12,10 @@ constexpr int kBuckets = 64;
 // Work lists.  The plan kernels fill the first three; solve kernels append
 // to the last two.
 enum RidgeClass {
-  CLS_SMALL = 0,    // FP64, 24 < (p+1) <= 48: 4x4 register tiles + row slices
+  CLS_SMALL = 0,    // FP64, 24 < (p+1) <= 48: warps alone, FP64 MMA Grams (ridge_dmma.cu)
   CLS_LARGE = 1,    // FP64, (p+1) > 48: 8x8 register tiles
-  CLS_TENSOR = 2,   // mixed form, p > 32: tcgen05 split-product Gram
-  CLS_WARP = 3,     // FP64, (p+1) <= 24: one warp per system
+  CLS_TENSOR = 2,   // mixed form, p at or above its threshold: tcgen05 split-product Gram
+  CLS_WARP = 3,     // FP64, (p+1) <= 24: as CLS_SMALL, narrower blocks and more warps
   CLS_QR = 4,       // auto solver fallback: Householder QR
   CLS_RESOLVE = 5,  // mixed form systems re-solved by the FP64 form
   kClasses = 6
@@ -23,7 +23,28 @@ enum RidgeClass {
 constexpr int kPlanClasses = 4;
 constexpr int kWarpMaxAug = 24;
 constexpr int kSmallMaxAug = 48;
-constexpr int kTensorMinP = 33;
+constexpr int kTensorMinP = 33;  // smallest p the tensor-core kernel takes
+// The mixed form's default threshold: below it the FP64 MMA kernel is the
+// faster one as well as the more exact (p = 45, 1,675 rows a system: 0.09 us
+// a system against 2.0 us on the tensor-core kernel).
+constexpr int kTensorDefaultP = kSmallMaxAug;
+// Split systems (see ridge_dmma.cu): units per system at most, batches above
+// kSplitMaxCount systems are not split (they fill every warp by number).
+constexpr int kMaxUnits = 256;
+constexpr int kSplitMaxCount = 16384;
+constexpr size_t kSplitPoolBytes = (size_t)256 << 20;
+constexpr int kSplitRecs = 4096;
+constexpr int kSplitItems = 32768;
+
+// Rows per unit of a system of n rows and augmented width pa: fixed by the
+// system alone, so that its sums do not depend on who forms them.  At least
+// 256 rows (a Gram is then added for every 64 MMA steps that form it), and at
+// most kMaxUnits units (a 400,000-row node of 45 features: units of 1,568
+// rows; twice as long ones left its last warps 0.4 ms behind the others).
+__host__ __device__ __forceinline__ int64_t ridge_unit_rows(int64_t n) {
+  const int64_t u = ((n + kMaxUnits - 1) / kMaxUnits + 31) / 32 * 32;
+  return u > 256 ? u : 256;
+}
 
 struct RidgeArgs {
   int64_t K;
@@ -53,6 +74,13 @@ struct RidgeArgs {
   int64_t gram_stride;
 };
 
+// A system split over several warps: its pool slots hold nseg packed Grams.
+struct SplitRec {
+  int64_t base;  // first double in the pool
+  int32_t k, nseg;
+  int32_t bad, pad;
+};
+
 struct RidgeLists {
   int32_t* count;   // [kClasses]
   int32_t* cursor;  // [kClasses]
@@ -61,6 +89,17 @@ struct RidgeLists {
   int32_t* err;     // [1] device-side error flag (bounded wait gave up)
   double* lambda;   // [K] effective ridge, kept for the QR fallback
   int32_t* list;    // [kClasses][K]
+  // split systems of CLS_WARP (0) and CLS_SMALL (1)
+  unsigned long long* cost;   // [2] summed row costs of the class
+  unsigned long long* pool_used;  // doubles taken from the pool
+  int32_t* nrec;    // records taken
+  int32_t* nitems;  // [2] queue entries: (record, first unit, units)
+  SplitRec* recs;
+  int4* items;      // [2][item_cap]
+  double* pool;
+  int64_t pool_cap; // doubles; 0: no system is split
+  int32_t rec_cap, item_cap;
+  int32_t workers[2];  // warps the class's kernel keeps resident
 };
 
 struct RidgeItem {
@@ -230,9 +269,19 @@ __device__ __forceinline__ int tile_row(int t) {
   return I;
 }
 
-// Host-side launch helpers (ridge.cu / ridge_tc.cu / ridge_warp.cu).
+// D (8x8, two doubles per lane) += A (8x4) * B (4x8) in FP64 on the tensor
+// cores.  Lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4) + {0,1}].
+__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// Host-side launch helpers (ridge.cu / ridge_tc.cu / ridge_dmma.cu).
 int launch_ridge_tensor(const RidgeArgs& a, const RidgeLists& L, cudaStream_t stream);
-int launch_ridge_warp(const RidgeArgs& a, const RidgeLists& L, cudaStream_t stream);
+int launch_ridge_dmma(const RidgeArgs& a, const RidgeLists& L, int cls, cudaStream_t stream);
+int launch_ridge_split_finish(const RidgeArgs& a, const RidgeLists& L, cudaStream_t stream);
+int ridge_dmma_ctas(int cls);
 int device_sm_count();
 
 }  // namespace art

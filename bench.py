@@ -858,14 +858,14 @@ def run_b200(args):
     from art.models import kind_feature_count
 
     p_all = np.array([kind_feature_count(int(a), int(b)) for a, b in zip(wl.dims, wl.kinds)])
-    if name == "ridge_warp":
+    thr = args.tensor_min_features or (tuned["tensor_min_features"] if tuned else 48)
+    if "dmma<3>" in name:
         cls_idx = np.flatnonzero(p_all + 1 <= 24)
-    elif "fp64<4>" in name:
-        cls_idx = np.flatnonzero((p_all + 1 > 24) & (p_all + 1 <= 48) & ((p_all < 33) | (args.precision == "fp64")))
+    elif "dmma<6>" in name:
+        cls_idx = np.flatnonzero((p_all + 1 > 24) & (p_all + 1 <= 48) & ((p_all < thr) | (args.precision == "fp64")))
     elif "fp64<8>" in name:
         cls_idx = np.flatnonzero(p_all + 1 > 48) if args.precision == "fp64" else np.flatnonzero(info & N.INFO_FP64_RESOLVE)
     else:
-        thr = args.tensor_min_features or (tuned["tensor_min_features"] if tuned else 33)
         cls_idx = np.flatnonzero(p_all >= thr)
     flops, nbytes = algorithmic(wl, cls_idx)
     achieved_gbs = nbytes / (per_launch_ms / 1000.0) / 1e9

@@ -138,7 +138,7 @@ typedef struct ArtRidgeProblem {
   uint32_t options;       /* ART_RIDGE_OPT_* bits                           */
   int32_t tensor_min_features; /* mixed form: systems with p >= this go to the
                                   tensor-core kernel, smaller ones to the FP64
-                                  kernels (0: 33; > 160: none)               */
+                                  kernels (0: 48; > 160: none)               */
 } ArtRidgeProblem;
 
 /* Mixed form: factor the tensor-core Gram in FP64 instead of FP32 (fewer
@@ -155,6 +155,9 @@ typedef struct ArtRidgeResult {
   uint32_t* info;          /* device [K] ART_INFO_* (may be NULL)          */
 } ArtRidgeResult;
 
+/* Scratch of one call.  For up to 16,384 systems it includes room (at most
+ * 256 MiB) to split large systems over many warps; a call given less, down to
+ * the lists alone, splits fewer of them, with the same results.              */
 ART_API size_t art_ridge_workspace_size(int64_t count, int32_t max_features);
 /* Weighted Grams only, by the mixed form's tensor-core path: for every system
  * with 33 <= p <= 160 and d <= ART_MAX_DIM, G' = sum_k q_k phi_k phi_k^T from
