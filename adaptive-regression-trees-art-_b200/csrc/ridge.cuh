@@ -25,8 +25,8 @@ constexpr int kWarpMaxAug = 24;
 constexpr int kSmallMaxAug = 48;
 constexpr int kTensorMinP = 33;  // smallest p the tensor-core kernel takes
 // The mixed form's default threshold: below it the FP64 MMA kernel is the
-// faster one as well as the more exact (p = 45, 1,675 rows a system: 0.09 us
-// a system against 2.0 us on the tensor-core kernel).
+// faster one as well as the more exact (2,048 weighted systems of 306 to 8,192
+// rows and 45 features: 0.54 ms against 3.6 ms on the tensor-core kernel).
 constexpr int kTensorDefaultP = kSmallMaxAug;
 // Split systems (see ridge_dmma.cu): units per system at most, batches above
 // kSplitMaxCount systems are not split (they fill every warp by number).

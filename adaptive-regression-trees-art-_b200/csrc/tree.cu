@@ -7,72 +7,187 @@
 // arithmetic for the rare scores within its error bound); numpy's own
 // rounded X @ w - z can disagree only where its rounding error exceeds
 // |w . x - z|.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace art {
 namespace {
 
-constexpr int kPartThreads = 256;
+// Both level kernels below give a node to a cluster of CTAs, since the nodes of
+// a level differ by a factor of a thousand in rows and one CTA reads only
+// about 50 GB/s.  The cluster's size follows the number of nodes (the more
+// nodes, the less a large one matters); what is added, and in which order,
+// follows the node's own row count, so results do not depend on it.
+// 307 nodes of 450 to 400,000 rows, d = 2 to 32 (1.7 GB): partition 14.5 ->
+// 0.59 ms, residuals 9.6 -> 0.65 ms against one CTA a node (2.6-2.9 TB/s of x
+// read once; before, the partition read it twice).
+constexpr int kLevelThreads = 256;
+constexpr int kLevelWarps = kLevelThreads / 32;
+constexpr int kMaxRanks = 16;  // CTAs of a cluster, and partial sums of a node, at most
 
-__global__ void __launch_bounds__(kPartThreads)
+int level_cluster(int64_t count) { return count <= 512 ? 16 : (count <= 2048 ? 8 : (count <= 8192 ? 4 : 1)); }
+
+// Eight doubles x[i .. i + 8) of a row of d (zeros past its end).  vec: 4 =
+// rows of whole 32-byte sectors (one 256-bit load each), 2 = of 16-byte
+// pairs, 1 = single doubles.  A thread reads its own row: every load moves
+// whole sectors, and a row's loads are all in flight together.
+__device__ __forceinline__ void load8(const double* x, int i, int d, int vec, double (&v)[8]) {
+  if (vec == 4) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (i + 4 * q < d) {
+        asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(v[4 * q]), "=d"(v[4 * q + 1]), "=d"(v[4 * q + 2]), "=d"(v[4 * q + 3])
+                     : "l"(x + i + 4 * q));
+      } else {
+        v[4 * q] = v[4 * q + 1] = v[4 * q + 2] = v[4 * q + 3] = 0.0;
+      }
+    }
+  } else if (vec == 2) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double2 t = i + 2 * q < d ? __ldg((const double2*)(x + i + 2 * q)) : make_double2(0.0, 0.0);
+      v[2 * q] = t.x;
+      v[2 * q + 1] = t.y;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = i + q < d ? __ldg(x + i + q) : 0.0;
+  }
+}
+__device__ __forceinline__ int row_vec(const double* x, int d) {
+  const uintptr_t at = (uintptr_t)x;
+  return (d & 3) == 0 && (at & 31) == 0 ? 4 : ((d & 1) == 0 && (at & 15) == 0 ? 2 : 1);
+}
+
+// right_side, decided by the plain score where that is further from zero
+// than its error bound (gamma_{d+1} times sum |x_i w_i| + |z|, taken twice);
+// w is zero-padded to a multiple of eight.  Two FMAs an input against eleven
+// operations for the compensated score, which still decides the rest, NaN
+// and infinite scores and products near underflow among them.
+__device__ __forceinline__ bool row_side(const double* xr, const double* w, int d, double z, int vec) {
+  double s = 0.0, mag = 0.0;
+#pragma unroll 4
+  for (int i = 0; i < d; i += 8) {
+    double v[8];
+    load8(xr, i, d, vec, v);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      s = fma(v[q], w[i + q], s);
+      mag = fma(fabs(v[q]), fabs(w[i + q]), mag);
+    }
+  }
+  s = __dsub_rn(s, z);
+  mag = __dadd_rn(mag, fabs(z));
+  const double bound = 2.220446049250313e-16 * (d + 4) * mag;
+  if (fabs(s) > bound && mag > 1e-280) return s >= 0.0;
+  return right_side(xr, w, d, z);
+}
+
+// Stable partition.  CTA r of a node's cluster takes the r-th range of its
+// rows: it reads x once, keeps the sides as a bit mask in shared memory, learns
+// the other ranges' right counts through distributed shared memory, and
+// scatters its row numbers to their places.  Rows past the mask's capacity
+// (2^18 a CTA) have their sides formed a second time.
+constexpr int kMaskWords = 8192;
+__global__ void __launch_bounds__(kLevelThreads)
     partition_kernel(ArtSegments seg, const double* x, const double* theta, int64_t ts,
                      const int8_t* split, int64_t* perm, int32_t* n_right) {
-  const int k = blockIdx.x;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
+  const int64_t k = blockIdx.x / csize;
   const int64_t r0 = seg.row_offsets[k], n = seg.row_offsets[k + 1] - r0;
   const int64_t xoff = seg.x_offsets[k];
   const int d = seg.dims[k];
   const bool do_split = split == nullptr || split[k] != 0;
-  __shared__ double w[ART_MAX_DIM + 1];
-  __shared__ int64_t s_base_left, s_base_right;
-  __shared__ int warp_tot[kPartThreads / 32];
+  extern __shared__ unsigned mask[];
+  __shared__ double w[ART_MAX_DIM + 8];
+  __shared__ int64_t s_right;
+  __shared__ int s_warp[kLevelWarps];
+  __shared__ int pre[kLevelThreads];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i <= d; i += kPartThreads) w[i] = theta[(int64_t)k * ts + i];
+  for (int i = tid; i < ART_MAX_DIM + 8; i += kLevelThreads) w[i] = i < d ? theta[k * ts + i] : 0.0;
+  const double z = theta[k * ts + d];
+  const double* xk = x + xoff;
+  const int vec = row_vec(xk, d);
+  const int64_t span = ((n + csize - 1) / csize + kLevelThreads - 1) / kLevelThreads * kLevelThreads;
+  const int64_t a = min(n, span * crank), b = min(n, a + span);  // this CTA's rows
   __syncthreads();
-  // pass 1: count right rows
   int local = 0;
-  if (do_split)
-    for (int64_t r = tid; r < n; r += kPartThreads) {
-      local += right_side(x + xoff + r * d, w, d, w[d]) ? 1 : 0;
+#pragma unroll 2
+  for (int64_t base = a; base < b; base += kLevelThreads) {
+    const int64_t r = base + tid;
+    const bool right = do_split && r < b && row_side(xk + r * d, w, d, z, vec);
+    const unsigned m = __ballot_sync(0xffffffffu, right);
+    const int64_t word = (base - a) / 32 + warp;
+    if (lane == 0) {
+      local += __popc(m);
+      if (word < kMaskWords) mask[word] = m;
     }
-  int tot = warp_sum(local);
-  if (lane == 0) warp_tot[warp] = tot;
+  }
+  if (lane == 0) s_warp[warp] = local;
   __syncthreads();
   if (tid == 0) {
     int64_t t = 0;
-    for (int i = 0; i < kPartThreads / 32; ++i) t += warp_tot[i];
-    s_base_left = 0;
-    s_base_right = n - t;
-    if (n_right) n_right[k] = (int32_t)t;
+    for (int i = 0; i < kLevelWarps; ++i) t += s_warp[i];
+    s_right = t;
   }
-  __syncthreads();
-  // pass 2: stable scatter in tiles of kPartThreads rows
-  for (int64_t base = 0; base < n; base += kPartThreads) {
-    const int64_t r = base + tid;
-    int right = 0;
-    if (r < n && do_split) right = right_side(x + xoff + r * d, w, d, w[d]) ? 1 : 0;
-    const unsigned bal = __ballot_sync(0xffffffffu, right);
-    const unsigned inb = __ballot_sync(0xffffffffu, r < n);
-    const int wr = __popc(bal), wl = __popc(inb & ~bal);
-    __shared__ int s_wr[kPartThreads / 32], s_wl[kPartThreads / 32];
-    if (lane == 0) { s_wr[warp] = wr; s_wl[warp] = wl; }
-    __syncthreads();
-    int pre_r = 0, pre_l = 0, tile_r = 0, tile_l = 0;
-    for (int i = 0; i < kPartThreads / 32; ++i) {
-      if (i < warp) { pre_r += s_wr[i]; pre_l += s_wl[i]; }
-      tile_r += s_wr[i];
-      tile_l += s_wl[i];
-    }
-    const unsigned lt = (1u << lane) - 1u;
-    if (r < n) {
-      int64_t pos;
-      if (right) pos = s_base_right + pre_r + __popc(bal & lt);
-      else pos = s_base_left + pre_l + __popc(inb & ~bal & lt);
-      perm[r0 + pos] = r0 + r;
-    }
-    __syncthreads();
-    if (tid == 0) { s_base_right += tile_r; s_base_left += tile_l; }
-    __syncthreads();
+  cluster.sync();
+  int64_t before = 0, total = 0;  // right rows of the ranges before this one, and of all
+  for (int c = 0; c < csize; ++c) {
+    const int64_t v = *cluster.map_shared_rank(&s_right, c);
+    if (c < crank) before += v;
+    total += v;
   }
+  if (n_right && crank == 0 && tid == 0) n_right[k] = (int32_t)total;
+  int64_t left = a - before, rgt = n - total + before;  // next places of this range
+  for (int64_t base = a; base < b; base += 32 * kLevelThreads) {
+    const int64_t words = min((int64_t)kLevelThreads, (b - base + 31) / 32);
+    // exclusive prefix of the right counts of up to 256 words
+    auto word_at = [&](int64_t q, int64_t row) -> unsigned {
+      const int64_t at = (base - a) / 32 + q;
+      if (at < kMaskWords) return mask[at];
+      unsigned m = 0;
+      for (int j = 0; j < 32 && row + j < b; ++j)
+        if (do_split && row_side(xk + (row + j) * d, w, d, z, vec)) m |= 1u << j;
+      return m;
+    };
+    const unsigned mine = tid < words ? word_at(tid, base + 32 * tid) : 0u;
+    const int cnt = __popc(mine);
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    __syncthreads();
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int wbase = 0, all = 0;
+    for (int i = 0; i < kLevelWarps; ++i) {
+      if (i < warp) wbase += s_warp[i];
+      all += s_warp[i];
+    }
+    pre[tid] = wbase + incl - cnt;
+    __syncwarp();
+    for (int q = 0; q < 32; ++q) {  // this warp's 32 words, a row per lane
+      const int wq = 32 * warp + q;
+      if (wq >= words) break;
+      const unsigned m = __shfl_sync(0xffffffffu, mine, q);
+      const int64_t r = base + 32 * (int64_t)wq + lane;
+      if (r < b) {
+        const int ahead = pre[wq] + __popc(m & ((1u << lane) - 1u));
+        const int64_t pos = (m >> lane) & 1u ? rgt + ahead : left + (32 * wq + lane - ahead);
+        perm[r0 + pos] = r0 + r;
+      }
+    }
+    rgt += all;
+    left += min((int64_t)32 * kLevelThreads, b - base) - all;
+  }
+  cluster.sync();  // the counts stay until every CTA has read them
 }
 
 __device__ inline double leaf_predict(const double* xr, int d, int kind, const double* c) {
@@ -102,55 +217,140 @@ __global__ void predict_kernel(int d, int64_t n_nodes, const int32_t* child, con
   if (pred) pred[i] = leaf_predict(xr, d, features[node], coef + (int64_t)node * cs);
 }
 
-// Per segment: sum of squared residuals of phi(x) . beta and sum of y^2.
-// One CTA per segment; each thread walks its rows in order, then a fixed
-// shared-memory tree sums the threads (deterministic for a given segment).
-constexpr int kResThreads = 256;
-__global__ void __launch_bounds__(kResThreads)
+// Per segment: sum of squared residuals of phi(x) . beta and sum of y^2.  A
+// node's rows are cut into up to kMaxRanks ranges, fixed by its row count;
+// each range is one CTA's sum (threads in row order, then a fixed tree), and
+// the ranges are added in order.
+template <int DP>
+__device__ __forceinline__ double quad_predict(const double* xr, const double* q, int d, int vec) {
+  // nested form of the quadratic: x_i (b_i + sum_{j >= i} b_ij x_j), the
+  // coefficients zero-padded to DP inputs: [b_0 | DP linear | DP (DP + 1) / 2]
+  double v[DP];
+#pragma unroll
+  for (int i = 0; i < DP; i += 8) {
+    double t[8];
+    load8(xr, i, d, vec, t);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[i + u] = t[u];
+  }
+  double s = q[0];
+  int f = 1 + DP;
+#pragma unroll
+  for (int i = 0; i < DP; ++i) {
+    double t = q[1 + i];
+#pragma unroll
+    for (int j = i; j < DP; ++j) t = fma(v[j], q[f++], t);
+    s = fma(v[i], t, s);
+  }
+  return s;
+}
+
+__device__ __forceinline__ double linear_predict(const double* xr, const double* q, int d, int vec) {
+  double s = q[0];
+#pragma unroll 4
+  for (int i = 0; i < d; i += 8) {
+    double v[8];
+    load8(xr, i, d, vec, v);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s = fma(v[u], q[1 + i + u], s);
+  }
+  return s;
+}
+
+__global__ void __launch_bounds__(kLevelThreads)
     residual_kernel(ArtSegments seg, const double* x, const double* y, const double* beta,
                     int64_t bs, double* sse, double* ssy) {
-  const int k = blockIdx.x;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
+  const int64_t k = blockIdx.x / csize;
   const int64_t r0 = seg.row_offsets[k], n = seg.row_offsets[k + 1] - r0;
   const int64_t xoff = seg.x_offsets[k];
   const int d = seg.dims[k], kind = seg.features[k];
   const int p = feature_count(d, kind);
-  __shared__ double b[ART_MAX_FEATURES];
-  __shared__ int16_t fa[ART_MAX_FEATURES], fb[ART_MAX_FEATURES];
-  __shared__ double red[2][kResThreads];
-  for (int f = threadIdx.x; f < p; f += kResThreads) {
+  // coefficients by position: constant, inputs (zero-padded), products
+  __shared__ double q[ART_MAX_FEATURES + 8 + 16];
+  __shared__ double part[2][kMaxRanks];
+  __shared__ double red[2][kLevelWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool quad = kind == ART_FEATURES_POLY2 || kind == ART_FEATURES_POLY2_NOBIAS;
+  const int dp = quad ? (d <= 8 ? 8 : 16) : d;
+  for (int i = tid; i < ART_MAX_FEATURES + 8 + 16; i += kLevelThreads) q[i] = 0.0;
+  __syncthreads();
+  for (int f = tid; f < p; f += kLevelThreads) {
     int u, v;
     feature_factors(d, kind, f, u, v);
-    fa[f] = (int16_t)u;
-    fb[f] = (int16_t)v;
-    b[f] = beta[(int64_t)k * bs + f];
+    int at;
+    if (u < 0) at = 0;
+    else if (v < 0) at = 1 + u;
+    else at = 1 + dp + u * dp - u * (u - 1) / 2 + (v - u);
+    if (at < ART_MAX_FEATURES + 24) q[at] = beta[k * bs + f];
   }
   __syncthreads();
-  double s_e = 0.0, s_y = 0.0;
-  for (int64_t r = threadIdx.x; r < n; r += kResThreads) {
-    const double* xr = x + xoff + r * d;
-    double pred = 0.0;
-    for (int f = 0; f < p; ++f) {
-      const int u = fa[f], v = fb[f];
-      pred = fma((u < 0 ? 1.0 : xr[u]) * (v < 0 ? 1.0 : xr[v]), b[f], pred);
+  const double* xk = x + xoff;
+  const int vec = row_vec(xk, d);
+  const int ranks = (int)min((int64_t)kMaxRanks, (n + 1023) / 1024);
+  const int64_t span = ranks ? (n + ranks - 1) / ranks : 0;
+  for (int v = crank; v < ranks; v += csize) {
+    const int64_t a = span * v, b = min(n, a + span);
+    double s_e = 0.0, s_y = 0.0;
+#pragma unroll 2
+    for (int64_t r = a + tid; r < b; r += kLevelThreads) {
+      const double* xr = xk + r * d;
+      const double yv = __ldg(y + r0 + r);
+      double pred;
+      if (!quad) pred = linear_predict(xr, q, d, vec);
+      else if (dp == 8) pred = quad_predict<8>(xr, q, d, vec);
+      else pred = quad_predict<16>(xr, q, d, vec);
+      const double e = yv - pred;
+      s_e = fma(e, e, s_e);
+      s_y = fma(yv, yv, s_y);
     }
-    const double yv = y[r0 + r], e = yv - pred;
-    s_e = fma(e, e, s_e);
-    s_y = fma(yv, yv, s_y);
-  }
-  red[0][threadIdx.x] = s_e;
-  red[1][threadIdx.x] = s_y;
-  __syncthreads();
-  for (int h = kResThreads / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h) {
-      red[0][threadIdx.x] += red[0][threadIdx.x + h];
-      red[1][threadIdx.x] += red[1][threadIdx.x + h];
+    s_e = warp_sum(s_e);
+    s_y = warp_sum(s_y);
+    if (lane == 0) { red[0][warp] = s_e; red[1][warp] = s_y; }
+    __syncthreads();
+    if (tid < 2) {
+      double t = 0.0;
+      for (int i = 0; i < kLevelWarps; ++i) t += red[tid][i];
+      *cluster.map_shared_rank(&part[tid][v], 0) = t;
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    sse[k] = red[0][0];
-    ssy[k] = red[1][0];
+  cluster.sync();
+  if (crank == 0 && tid < 2) {
+    double t = 0.0;
+    for (int v = 0; v < ranks; ++v) t += part[tid][v];
+    (tid ? ssy : sse)[k] = t;
   }
+}
+
+template <typename... P, typename... A>
+int launch_level(void (*kern)(P...), int64_t count, size_t smem, cudaStream_t s, const char* what, A... args) {
+  const int c = level_cluster(count);
+  if ((c > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+      (smem && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess))
+    return check_launch(what);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)c;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(count * c));
+  cfg.blockDim = dim3(kLevelThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  prof_begin(what, s);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  prof_end(s);
+  count_launch();
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    set_error("%s: %s", what, cudaGetErrorString(e));
+    return ART_E_LAUNCH;
+  }
+  return check_launch(what);
 }
 
 }  // namespace
@@ -170,12 +370,8 @@ extern "C" int art_segment_residuals(const ArtSegments* seg, const double* x, co
     return ART_E_INVALID;
   }
   if (seg->count > 0x7fffffffll) { set_error("art_segment_residuals: too many segments"); return ART_E_UNSUPPORTED; }
-  prof_begin("segment_residuals", (cudaStream_t)stream);
-  residual_kernel<<<(unsigned)seg->count, kResThreads, 0, (cudaStream_t)stream>>>(*seg, x, y, beta, beta_stride,
-                                                                                  sse, ssy);
-  prof_end((cudaStream_t)stream);
-  count_launch();
-  return check_launch("art_segment_residuals");
+  return launch_level(residual_kernel, seg->count, 0, (cudaStream_t)stream, "segment_residuals", *seg, x, y, beta,
+                      beta_stride, sse, ssy);
 }
 
 extern "C" int art_partition_rows(const ArtSegments* seg, const double* x, const double* theta,
@@ -186,12 +382,8 @@ extern "C" int art_partition_rows(const ArtSegments* seg, const double* x, const
   if (seg->count < 0 || seg->count > 0x7fffffff) { set_error("art_partition_rows: bad count"); return ART_E_INVALID; }
   if (seg->count == 0) return ART_OK;
   if (theta_stride < 2) { set_error("art_partition_rows: theta_stride too small"); return ART_E_INVALID; }
-  prof_begin("partition_rows", (cudaStream_t)stream);
-  partition_kernel<<<(unsigned)seg->count, kPartThreads, 0, (cudaStream_t)stream>>>(
-      *seg, x, theta, theta_stride, split, perm, n_right);
-  prof_end((cudaStream_t)stream);
-  count_launch();
-  return check_launch("art_partition_rows");
+  return launch_level(partition_kernel, seg->count, kMaskWords * sizeof(unsigned), (cudaStream_t)stream,
+                      "partition_rows", *seg, x, theta, theta_stride, split, perm, n_right);
 }
 
 extern "C" int art_tree_predict(int32_t dim, int64_t n_nodes, const int32_t* child,
