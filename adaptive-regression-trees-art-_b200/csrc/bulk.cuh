@@ -80,6 +80,19 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       : "memory");
 }
 
+// Per-thread asynchronous copies global -> shared of 8 or 16 bytes (both
+// addresses aligned to the size); `live` off writes zeros.
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, bool live = true) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool live = true) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Waits for all but the newest group, or for all, of this thread's copies.
+__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
 // A byte range [src, src+bytes) widened to whole 16-byte granules.  Reading
 // a whole granule never leaves the page of its first valid byte, so the
 // widening is always mapped memory.

@@ -10,18 +10,36 @@
 //    _step_interval 540-564): unit directions, slack recomputed from x each
 //    step, |A u| > 1e-14 tests, samples at steps burn_in + k*thinning.
 //
-// Layout: a team of L lanes (L = next power of two >= ceil(d/2), L <= 32)
-// advances one chain; lane l owns coordinates 2l and 2l+1, so one Philox
-// block gives both of its normals.  Box rows (+e_i, -e_i) are applied
-// structurally: A u = +-u_i exactly, as in the reference's dense matmul.
-// Oblique rows are held in shared memory and reduced across the team.
+// A step has a part that depends on the chain's state (the chord bounds from
+// the slacks, the step, the new slacks) and a larger one that does not (the
+// draws, and the products A u of every oblique row with the direction).  A team
+// of TL lanes advances one chain, a block of SB steps at a time:
+//   1. the block's directions are drawn (or copied ahead of time, if injected)
+//      into shared memory, a Philox block per (step, coordinate pair);
+//   2. lane = step: A u for every row, four rows at a time, and the uniform;
+//   3. lane = constraint: the steps one after another, each lane holding the
+//      slacks of its coordinates and rows.  A step is a product with the
+//      reciprocal of A u (formed ahead, off the dependent path), a minimum and
+//      a maximum over the team, and the update.
+// What bounds it: for few chains the dependent path of part 3 (so a whole warp
+// per chain, the minima and maxima by integer redux.sync on the ordered bits),
+// for many chains instruction issue, 70 % of the slots (so teams of 8 or 16
+// lanes where the dimension allows).  Against a step that drew, multiplied and
+// divided in turn, bit for bit the same states: 61 chains of 2,100 steps in 4
+// dimensions 7.64 -> 0.46 ms, 16,384 chains of 1,000 steps in 8 dimensions
+// 4.05 -> 1.79 ms.
+// Box rows (+e_i, -e_i) are applied structurally: A u = +-u_i exactly, as in
+// the reference's dense matmul, and of a coordinate's two rows one bounds the
+// step from above and the other from below.
 #include <algorithm>
+
+#include "bulk.cuh"
 #include "common.cuh"
 
 namespace art {
 namespace {
 
-constexpr int kHarThreads = 256;
+constexpr int kHarThreads = 128;
 constexpr double kScalarParallelTol = 1e-14;  // sampling.py:552-553
 constexpr double kFeasTol = 1e-10;             // sampling.py:438, domain.py:40
 
@@ -45,109 +63,178 @@ struct HarArgs {
   uint64_t counter_base;
   double* samples;
   int32_t* status;
+  int cap;  // oblique rows a team has room for
 };
 
-template <int L>
-__device__ __forceinline__ double team_sum(double v) {
-#pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+// A chain of a thousand steps in eight dimensions amplifies a rounding by ten
+// orders of magnitude, so every operation that reaches the state keeps one
+// order and one rounding whatever the team: products are summed by coordinate
+// pairs in a halving tree (pair_tree), quotients are correctly rounded.
+
+// 1 / v within an ulp or two: the hardware's approximation and two
+// Newton-Raphson steps r <- r + r (1 - v r).
+__device__ __forceinline__ double newton_rcp(double v) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
+  r = fma(r, fma(-v, r, 1.0), r);
+  return fma(r, fma(-v, r, 1.0), r);
 }
-template <int L>
-__device__ __forceinline__ double team_max(double v) {
-#pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+// s / v rounded to nearest from y = newton_rcp(v): q = s y and one correction
+// by its residual s - q v (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 1990); what is rounded
+// last is within 2^-104 of the quotient.  y does not depend on the state, so
+// only these three operations are on a step's dependent path.
+__device__ __forceinline__ double quotient(double s, double v, double y) {
+  const double q = s * y;
+  return fma(fma(-q, v, s), y, q);
 }
-template <int L>
-__device__ __forceinline__ double team_min(double v) {
-#pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-template <int L>
-__device__ __forceinline__ int team_or(int v) {
-#pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+// The plain division, kept out of line: it is almost never needed.
+__device__ __noinline__ double divided(double s, double v) { return s / v; }
+// |v| in about [1e-288, 1e290], where the residual neither under- nor overflows
+__device__ __forceinline__ bool quotient_range(double v) {
+  return ((uint32_t)__double2hiint(v) & 0x7fffffffu) - 0x04200000u < 0x78000000u;
 }
 
-// Oblique rows of a team's polytope live in shared memory (team stride
-// MAXK * d + 1 doubles, odd, so the teams of a warp use different banks);
-// row r's slack, bound and direction product are kept by lane r % L only.
-template <int L, int MAXK>
-__host__ __device__ constexpr size_t har_team_stride(int d) { return (size_t)MAXK * d + 1; }
+// sum_i a_i v_i over d <= 2 H coordinates: a_2l v_2l + a_2l+1 v_2l+1 of each
+// pair, the pairs added in halves (l with l + H / 2, then H / 4, ...).  FMA: a
+// pair's first product rounded, the second not.  (With a single pair the
+// second is rounded, the first not.)
+template <int H, bool FMA = false>
+__device__ __forceinline__ double pair_tree(const double* a, const double* v, int d) {
+  double p[H];
+#pragma unroll
+  for (int l = 0; l < H; ++l) {
+    const double s = 2 * l < d ? __dmul_rn(a[2 * l], v[2 * l]) : 0.0;
+    const double t = 2 * l + 1 < d ? __dmul_rn(a[2 * l + 1], v[2 * l + 1]) : 0.0;
+    if (H == 1 && !FMA) p[l] = fma(a[0], v[0], t);
+    else p[l] = FMA && 2 * l + 1 < d ? fma(a[2 * l + 1], v[2 * l + 1], s) : __dadd_rn(s, t);
+  }
+#pragma unroll
+  for (int o = H / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int l = 0; l < o; ++l) p[l] = __dadd_rn(p[l], p[l + o]);
+  return p[0];
+}
 
-// Teams of 4 or more lanes on polytopes of up to 16 rows are held to two
-// resident CTAs per SM (128 registers a thread); narrower teams and longer
-// row lists take the registers they need.
-constexpr int har_min_ctas(int L, int MAXK) { return (L >= 4 && MAXK <= 16) ? 2 : 1; }
+// Minimum of hi and maximum of lo over the team's lanes.
+template <int TL>
+__device__ __forceinline__ void team_bounds(double& lo, double& hi) {
+  if constexpr (TL == 32) {
+    // doubles as ordered (signed high, unsigned low) words: two 32-bit warp
+    // reductions a bound instead of five rounds of 64-bit shuffles
+    auto key = [](double v, int& h, uint32_t& l) {
+      h = __double2hiint(v);
+      l = (uint32_t)__double2loint(v);
+      if (h < 0) { h ^= 0x7fffffff; l = ~l; }
+    };
+    auto value = [](int h, uint32_t l) {
+      if (h < 0) { h ^= 0x7fffffff; l = ~l; }
+      return __hiloint2double(h, (int)l);
+    };
+    int hh, lh;
+    uint32_t hl, ll;
+    key(hi, hh, hl);
+    key(lo, lh, ll);
+    const int mh = __reduce_min_sync(0xffffffffu, hh), xh = __reduce_max_sync(0xffffffffu, lh);
+    const uint32_t ml = __reduce_min_sync(0xffffffffu, hh == mh ? hl : 0xffffffffu);
+    const uint32_t xl = __reduce_max_sync(0xffffffffu, lh == xh ? ll : 0u);
+    hi = value(mh, ml);
+    lo = value(xh, xl);
+  } else {
+#pragma unroll
+    for (int o = TL / 2; o > 0; o >>= 1) {
+      const double h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
+      hi = h < hi ? h : hi;
+      lo = l > lo ? l : lo;
+    }
+  }
+}
+template <int TL>
+__device__ __forceinline__ bool team_any(bool v) {
+  const unsigned m = __ballot_sync(0xffffffffu, v);
+  const int lane = threadIdx.x & 31;
+  return ((m >> (lane / TL * TL)) & (TL == 32 ? 0xffffffffu : (1u << (TL & 31)) - 1u)) != 0;
+}
 
-template <int L, int MAXK>
-__global__ void __launch_bounds__(kHarThreads, har_min_ctas(L, MAXK)) har_kernel(HarArgs a) {
-  extern __shared__ double s_rows[];
-  constexpr int OWN = (MAXK + L - 1) / L;  // rows owned by each lane
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t chain_raw = gt / L;
-  const int lane = (int)(gt % L);
+// Shared memory of a team, in doubles: A [cap][d], the directions [bufs][SB][us],
+// the products [SB][as], the uniforms [bufs][SB], the state [d].  Odd strides
+// us and as put the lanes of part 2 (one step each) into different banks; the
+// team stride, 8 modulo 16, does the same for the teams of a warp.
+struct HarLayout {
+  int us, as, bufs;
+  int U, AU, UN, X, total;
+};
+__host__ __device__ inline HarLayout har_layout(int d, int cap, int SB, bool injected, bool maps) {
+  HarLayout L;
+  L.us = d | 1;
+  L.as = cap | 1;
+  L.bufs = injected || maps ? 2 : 1;  // the next block's draws in flight, or z beside u = M z
+  L.U = cap * d;
+  L.AU = L.U + L.bufs * SB * L.us;
+  L.UN = L.AU + SB * L.as;
+  L.X = L.UN + L.bufs * SB;
+  L.total = (L.X + d + 7) / 16 * 16 + 8;
+  while (L.total < L.X + d) L.total += 16;
+  return L;
+}
+
+template <int TL, int CPL, int RPL, int SB, int H, bool scalar>
+__global__ void __launch_bounds__(kHarThreads) har_kernel(HarArgs a) {
+  extern __shared__ double s_team[];
+  const int lane = (int)(threadIdx.x % TL);
+  const int64_t chain_raw = ((int64_t)blockIdx.x * kHarThreads + threadIdx.x) / TL;
   // Teams past the end keep running (masked) so that full-warp shuffles stay valid.
   const bool live = chain_raw < a.n_chains;
   const int64_t chain = live ? chain_raw : (a.n_chains - 1);
   const int d = a.d;
-  const int i0 = 2 * lane, i1 = 2 * lane + 1;
-  const bool h0 = i0 < d, h1 = i1 < d;
+  const bool injected = a.dirs != nullptr;
+  const HarLayout L = har_layout(d, a.cap, SB, injected, a.maps != nullptr && !injected);
+  double* As = s_team + (size_t)(threadIdx.x / TL) * L.total;
+  double* Us = As + L.U;
+  double* AUs = As + L.AU;
+  double* UNs = As + L.UN;
+  double* Xs = As + L.X;
   const int pj = a.polytope[chain];
   const int64_t rb = a.row_offsets[pj];
-  const int k = (int)(a.row_offsets[pj + 1] - rb);
-  const bool scalar = a.mode == ART_HAR_SCALAR;
+  int k = (int)(a.row_offsets[pj + 1] - rb);
   int status = 0;
-  if (k > MAXK) status = 3;
-  double x0 = h0 ? a.x[chain * d + i0] : 0.0;
-  double x1 = h1 ? a.x[chain * d + i1] : 0.0;
+  if (k > a.cap) { status = 3; k = 0; }
   const bool box = a.lo != nullptr;
-  double lo0 = 0, lo1 = 0, hi0 = 0, hi1 = 0;
-  if (box) {
-    lo0 = h0 ? a.lo[(int64_t)pj * d + i0] : 0.0;
-    lo1 = h1 ? a.lo[(int64_t)pj * d + i1] : 0.0;
-    hi0 = h0 ? a.hi[(int64_t)pj * d + i0] : 0.0;
-    hi1 = h1 ? a.hi[(int64_t)pj * d + i1] : 0.0;
+  const double inf = INFINITY;
+  // this lane's coordinates i = lane + TL m and rows r = lane + TL m
+  double x[CPL], shi[CPL], slo[CPL], hi_[CPL], lo_[CPL];
+  double so[RPL], br[RPL];
+#pragma unroll
+  for (int m = 0; m < CPL; ++m) {
+    const int i = lane + TL * m;
+    const bool own = i < d;
+    x[m] = own ? a.x[chain * d + i] : 0.0;
+    // a coordinate without a box never bounds the step: infinite slacks
+    lo_[m] = own && box ? a.lo[(int64_t)pj * d + i] : -inf;
+    hi_[m] = own && box ? a.hi[(int64_t)pj * d + i] : inf;
+    shi[m] = hi_[m] - x[m];
+    slo[m] = x[m] - lo_[m];
+    if (own) Xs[i] = x[m];
   }
-  double* Ar = s_rows + (size_t)(threadIdx.x / L) * har_team_stride<L, MAXK>(d);
-  for (int e = lane; e < MAXK * d; e += L) {
-    const int r = e / d, i = e - r * d;
-    Ar[e] = (r < k && status == 0) ? a.A[(rb + r) * d + i] : 0.0;
-  }
+  for (int e = lane; e < a.cap * d; e += TL) As[e] = e < k * d ? a.A[rb * d + e] : 0.0;
   __syncwarp();
-  // this lane's coefficient of row r on its two coordinates
-  auto arow = [&](int r, double v0, double v1) {
-    return (h0 ? Ar[r * d + i0] * v0 : 0.0) + (h1 ? Ar[r * d + i1] * v1 : 0.0);
+  auto row_slack = [&](int m) {  // b - A x of this lane's m-th row
+    const int r = lane + TL * m;
+    if (r >= k) return 0.0;
+    return __dsub_rn(br[m], pair_tree<H>(As + r * d, Xs, d));
   };
-  double br[OWN], so[OWN], au[OWN];
+  bool bad = false;
 #pragma unroll
-  for (int m = 0; m < OWN; ++m) {
-    const int r = m * L + lane;
-    br[m] = (r < MAXK && r < k && status == 0) ? a.b[rb + r] : 0.0;
-    so[m] = 0.0;
-    au[m] = 0.0;
-  }
-  // initial slacks s = b - A x (numba path: sampling.py:648)
-  double shi0 = hi0 - x0, shi1 = hi1 - x1, slo0 = x0 - lo0, slo1 = x1 - lo1;
-  int bad_start = 0;
-  if (box) {
-    if (h0 && (shi0 < -kFeasTol || slo0 < -kFeasTol)) bad_start = 1;
-    if (h1 && (shi1 < -kFeasTol || slo1 < -kFeasTol)) bad_start = 1;
+  for (int m = 0; m < RPL; ++m) {
+    const int r = lane + TL * m;
+    br[m] = r < k ? a.b[rb + r] : 0.0;
+    so[m] = row_slack(m);  // numba path: sampling.py:648
+    if (so[m] < -kFeasTol) bad = true;
   }
 #pragma unroll
-  for (int r = 0; r < MAXK; ++r) {
-    const double ax = team_sum<L>(arow(r, x0, x1));
-    if (r % L == lane) {
-      so[r / L] = br[r / L] - ax;
-      if (r < k && so[r / L] < -kFeasTol) bad_start = 1;
-    }
-  }
-  bad_start = team_or<L>(bad_start);
-  const int kwarp = __reduce_max_sync(0xffffffffu, status == 0 ? k : 0);
-  if (bad_start && status == 0) status = 2;
+  for (int m = 0; m < CPL; ++m)
+    if (shi[m] < -kFeasTol || slo[m] < -kFeasTol) bad = true;
+  if (team_any<TL>(bad) && status == 0) status = 2;
   const uint32_t key0 = a.seeds ? (uint32_t)a.seeds[chain] : 0u;
   const uint32_t key1 = a.seeds ? (uint32_t)(a.seeds[chain] >> 32) : 0u;
   const int total = a.burn_in + a.n_rounds * a.thinning;
@@ -158,154 +245,256 @@ __global__ void __launch_bounds__(kHarThreads, har_min_ctas(L, MAXK)) har_kernel
   // step of each thinning block after burn_in
   int keep_step = scalar ? a.burn_in : a.burn_in + a.thinning - 1;
   int keep_idx = 0;
-  // one step per iteration: the body is long, and unrolling it only grows the
-  // code the warps fetch
-#pragma unroll 1
-  for (int step = 0; step < total; ++step) {
-    double u0, u1;
-    if (a.dirs) {
-      const double* dp = a.dirs + (chain * total + step) * (int64_t)d;
-      u0 = h0 ? dp[i0] : 0.0;
-      u1 = h1 ? dp[i1] : 0.0;
+  constexpr int NP = TL / SB;               // lanes that share a step in part 2
+  const int st = lane % SB, part = lane / SB;
+  auto copy_block = [&](int s0, int buf) {  // injected draws of steps [s0, s0 + SB), in flight
+    const int ns = min(SB, total - s0);
+    const double* src = a.dirs + ((int64_t)chain * total + s0) * d;
+    double* dst = Us + buf * SB * L.us;
+    int r = lane / d, c = lane - r * d;
+    const int dr = TL / d, dc = TL - dr * d;
+    for (int e = lane; e < ns * d; e += TL) {
+      cp_async8(smem_u32(dst + r * L.us + c), src + e);
+      r += dr;
+      c += dc;
+      if (c >= d) { c -= d; ++r; }
+    }
+    if (!scalar && part == 0 && st < ns)
+      cp_async8(smem_u32(UNs + buf * SB + st), a.unif + (int64_t)chain * total + s0 + st);
+    cp_async_commit();
+  };
+  if (injected && total > 0) copy_block(0, 0);
+  for (int s0 = 0; s0 < total; s0 += SB) {
+    const int ns = min(SB, total - s0);
+    int buf = 0;
+    __syncwarp();
+    // ---- 1. directions
+    if (injected) {
+      buf = (s0 / SB) & 1;
+      if (s0 + SB < total) copy_block(s0 + SB, buf ^ 1);
+      else cp_async_commit();
+      cp_async_wait1();
     } else {
-      const uint64_t ctr = a.counter_base + (uint64_t)step;
-      Philox4 r = philox4x32_10((uint32_t)ctr, (uint32_t)(ctr >> 32), (uint32_t)lane, 0u, key0,
-                                key1);
-      normal_pair_f32(r, u0, u1);
-      if (!h0) u0 = 0.0;
-      if (!h1) u1 = 0.0;
-      if (a.maps) {  // covariance-shaped direction u = M z, z gathered across the team
+      buf = a.maps ? 1 : 0;
+      const int np = (d + 1) / 2;
+      double* z = Us + buf * SB * L.us;
+      for (int j = part; j < np; j += NP) {
+        const uint64_t ctr = a.counter_base + (uint64_t)(s0 + st);
+        const Philox4 r = philox4x32_10((uint32_t)ctr, (uint32_t)(ctr >> 32), (uint32_t)j, 0u, key0, key1);
+        double u0, u1;
+        normal_pair_f32(r, u0, u1);
+        z[st * L.us + 2 * j] = u0;
+        if (2 * j + 1 < d) z[st * L.us + 2 * j + 1] = u1;
+      }
+      if (a.maps) {  // covariance-shaped direction u = M z
+        __syncwarp();
         const double* M = a.maps + (int64_t)pj * d * d;
-        double m0 = 0.0, m1 = 0.0;
-        for (int j = 0; j < d; ++j) {
-          const double za = __shfl_sync(0xffffffffu, u0, j >> 1, L);
-          const double zb = __shfl_sync(0xffffffffu, u1, j >> 1, L);
-          const double zj = (j & 1) ? zb : za;
-          if (h0) m0 = fma(M[(int64_t)i0 * d + j], zj, m0);
-          if (h1) m1 = fma(M[(int64_t)i1 * d + j], zj, m1);
+        for (int i = part; i < d; i += NP) {
+          double t = 0.0;
+          for (int j = 0; j < d; ++j) t = fma(__ldg(M + (int64_t)i * d + j), z[st * L.us + j], t);
+          Us[st * L.us + i] = t;
         }
-        u0 = m0;
-        u1 = m1;
+        buf = 0;
       }
     }
-    bool skip = false;
+    double* U = Us + buf * SB * L.us;
+    double* UN = UNs + (injected ? buf * SB : 0);
+    __syncwarp();
+    // ---- 2. lane = step: unit direction (scalar mode), A u, the uniform
+    bool zero = false;
     if (scalar) {
-      const double nrm2 = team_sum<L>(u0 * u0 + u1 * u1);
-      const double nrm = sqrt(nrm2);
-      if (nrm == 0.0) skip = true;
-      else { u0 = u0 / nrm; u1 = u1 / nrm; }
-      // recompute slacks from x (sampling.py:548-550)
-      shi0 = hi0 - x0; shi1 = hi1 - x1; slo0 = x0 - lo0; slo1 = x1 - lo1;
-#pragma unroll
-      for (int r = 0; r < MAXK; ++r) {
-        const double ax = team_sum<L>(arow(r, x0, x1));
-        if (r % L == lane) so[r / L] = br[r / L] - ax;
+      const double n2 = pair_tree<H, true>(U + st * L.us, U + st * L.us, d);
+      const double nrm = sqrt(n2);
+      zero = st < ns && nrm == 0.0;
+      __syncwarp();
+      if (!zero)
+        for (int i = part; i < d; i += NP) U[st * L.us + i] = U[st * L.us + i] / nrm;
+      __syncwarp();
+    }
+    const unsigned zmask = __ballot_sync(0xffffffffu, zero) >> ((threadIdx.x & 31) / TL * TL);
+    if (part == 0 && st < ns) {
+      if (!injected) {
+        const uint64_t ctr = a.counter_base + (uint64_t)(s0 + st);
+        const Philox4 r = philox4x32_10((uint32_t)ctr, (uint32_t)(ctr >> 32), 0xFFFFFFFFu, 1u, key0, key1);
+        UN[st] = u01_closed_open(r.v[0], r.v[1]);
+      } else if (scalar) {
+        const int64_t at = ucur + st - __popc(zmask & ((1u << st) - 1u));
+        UN[st] = a.unif[(int64_t)chain * total + at];
       }
     }
-    // rows past the largest count in the warp are zero: skip them (a
-    // warp-uniform bound, so the team shuffles stay converged)
+    for (int r = part; r < k; r += NP) AUs[st * L.as + r] = pair_tree<H>(As + r * d, U + st * L.us, d);
+    __syncwarp();
+    // ---- 3. lane = constraint: the steps in order
+    double nu[CPL], niu[CPL], nau[RPL], nia[RPL], nun;
+    bool nodd;
+    const double* up_ = U + lane;
+    const double* ap_ = AUs + lane;
+    const double* np_ = UN;
+    auto fetch = [&]() {  // what the next step needs besides the state
+      bool odd = false;
 #pragma unroll
-    for (int r = 0; r < MAXK; ++r) {
-      if (r >= kwarp) break;
-      const double v = team_sum<L>(arow(r, u0, u1));
-      if (r % L == lane) au[r / L] = v;
-    }
-    if (!skip) {
-      const double pos_t = scalar ? kScalarParallelTol : 0.0;
-      double tlo = -INFINITY, thi = INFINITY;
-      int infeasible = 0;
-      auto box_row = [&](double slack, double prod) {
-        if (prod > pos_t) thi = fmin(thi, slack / prod);
-        else if (prod < -pos_t) tlo = fmax(tlo, slack / prod);
-        else if (scalar && slack < -kFeasTol) infeasible = 1;
-      };
-      if (box) {
-        if (h0) { box_row(shi0, u0); box_row(slo0, -u0); }
-        if (h1) { box_row(shi1, u1); box_row(slo1, -u1); }
+      for (int m = 0; m < CPL; ++m) {
+        nu[m] = lane + TL * m < d ? up_[TL * m] : 0.0;
+        niu[m] = newton_rcp(nu[m]);
+        odd |= nu[m] != 0.0 && !quotient_range(nu[m]);
       }
-      // each lane walks only the rows it owns (r = m L + lane); min and max
-      // do not depend on the order
 #pragma unroll
-      for (int m = 0; m < OWN; ++m) {
-        const int r = m * L + lane;
-        if (r < MAXK && r < k) box_row(so[m], au[m]);
+      for (int m = 0; m < RPL; ++m) {
+        nau[m] = lane + TL * m < k ? ap_[TL * m] : 0.0;
+        nia[m] = newton_rcp(nau[m]);
+        odd |= nau[m] != 0.0 && !quotient_range(nau[m]);
       }
-      tlo = team_max<L>(tlo);
-      thi = team_min<L>(thi);
-      infeasible = team_or<L>(infeasible);
-      if (status == 0 && (tlo > thi || infeasible)) status = 1;
-      double U;
-      if (a.unif) {
-        U = a.unif[chain * total + (scalar ? ucur : step)];
-      } else {
-        const uint64_t ctr = a.counter_base + (uint64_t)step;
-        Philox4 r = philox4x32_10((uint32_t)ctr, (uint32_t)(ctr >> 32), 0xFFFFFFFFu, 1u, key0,
-                                  key1);
-        U = u01_closed_open(r.v[0], r.v[1]);
-      }
-      ++ucur;
-      // Separate roundings (no FMA contraction), as numpy/numba evaluate them.
-      const double t = __dadd_rn(tlo, __dmul_rn(U, __dsub_rn(thi, tlo)));
-      if (status == 0) {
-        x0 = __dadd_rn(x0, __dmul_rn(t, u0));
-        x1 = __dadd_rn(x1, __dmul_rn(t, u1));
-        if (!scalar) {
-          shi0 = __dsub_rn(shi0, __dmul_rn(t, u0));
-          shi1 = __dsub_rn(shi1, __dmul_rn(t, u1));
-          slo0 = __dsub_rn(slo0, __dmul_rn(t, -u0));
-          slo1 = __dsub_rn(slo1, __dmul_rn(t, -u1));
+      nun = *np_;
+      // divisors outside the quotient's range (denormal directions): the
+      // step divides
+      nodd = __any_sync(0xffffffffu, odd);
+    };
+    fetch();
+#pragma unroll 2
+    for (int j = 0; j < ns; ++j) {
+      // a zero direction moves nothing (scalar mode skips the step; control
+      // flow stays the same for the warp's other teams)
+      const bool skip = scalar && ((zmask >> j) & 1u);
+      double u_[CPL], iu[CPL], au[RPL], ia[RPL];
 #pragma unroll
-          for (int m = 0; m < OWN; ++m) so[m] = __dsub_rn(so[m], __dmul_rn(t, au[m]));
+      for (int m = 0; m < CPL; ++m) { u_[m] = nu[m]; iu[m] = niu[m]; }
+#pragma unroll
+      for (int m = 0; m < RPL; ++m) { au[m] = nau[m]; ia[m] = nia[m]; }
+      const double un = nun;
+      const bool divide = nodd;
+      double thi = inf, tlo = -inf;
+      bool infeasible = false;
+      if constexpr (scalar) {  // slacks from x (sampling.py:548-550)
+#pragma unroll
+        for (int m = 0; m < RPL; ++m) so[m] = row_slack(m);
+#pragma unroll
+        for (int m = 0; m < CPL; ++m) { shi[m] = hi_[m] - x[m]; slo[m] = x[m] - lo_[m]; }
+      }
+      // A NaN quotient bounds nothing: that of an infinite slack (no box), of a
+      // zero product (its reciprocal is NaN), or, in scalar mode, of a product
+      // within the parallel tolerance (made NaN here).
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) {
+        double y = iu[m];
+        if constexpr (scalar) {
+          if (!(fabs(u_[m]) > kScalarParallelTol)) {
+            y = __longlong_as_double(0x7ff8000000000000ll);
+            infeasible |= shi[m] < -kFeasTol || slo[m] < -kFeasTol;
+          }
         }
+        double ra = quotient(shi[m], u_[m], y), rb_ = -quotient(slo[m], u_[m], y);
+        if (divide && y == y) { ra = divided(shi[m], u_[m]); rb_ = -divided(slo[m], u_[m]); }
+        const bool neg = __double2hiint(u_[m]) < 0;
+        const double h = neg ? rb_ : ra, l = neg ? ra : rb_;
+        thi = h < thi ? h : thi;
+        tlo = l > tlo ? l : tlo;
+      }
+#pragma unroll
+      for (int m = 0; m < RPL; ++m) {
+        double y = ia[m];
+        if constexpr (scalar) {
+          if (!(fabs(au[m]) > kScalarParallelTol)) {
+            y = __longlong_as_double(0x7ff8000000000000ll);
+            infeasible |= so[m] < -kFeasTol;
+          }
+        }
+        double r = quotient(so[m], au[m], y);
+        if (divide && y == y) r = divided(so[m], au[m]);
+        const bool neg = __double2hiint(au[m]) < 0;
+        if (!neg && r < thi) thi = r;
+        if (neg && r > tlo) tlo = r;
+      }
+      if (j + 1 < ns) {
+        up_ += L.us;
+        ap_ += L.as;
+        ++np_;
+      }
+      fetch();  // issued while the bounds travel
+      team_bounds<TL>(tlo, thi);
+      if constexpr (scalar) infeasible = team_any<TL>(infeasible);
+      if (status == 0 && !skip && (tlo > thi || infeasible)) status = 1;
+      // Separate roundings (no FMA contraction), as numpy/numba evaluate them.
+      const double t = __dadd_rn(tlo, __dmul_rn(un, __dsub_rn(thi, tlo)));
+      if (status == 0 && !skip) {
+#pragma unroll
+        for (int m = 0; m < CPL; ++m) {
+          const double tu = __dmul_rn(t, u_[m]);
+          x[m] = __dadd_rn(x[m], tu);
+          shi[m] = __dsub_rn(shi[m], tu);
+          slo[m] = __dadd_rn(slo[m], tu);
+        }
+#pragma unroll
+        for (int m = 0; m < RPL; ++m) so[m] = __dsub_rn(so[m], __dmul_rn(t, au[m]));
+      }
+      if constexpr (scalar) {
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < CPL; ++m)
+          if (lane + TL * m < d) Xs[lane + TL * m] = x[m];
+        __syncwarp();
+      }
+      // sample bookkeeping
+      if (s0 + j == keep_step) {
+        if (!skip && keep_idx < a.n_rounds && live) {
+          double* sp = a.samples + ((int64_t)keep_idx * C + chain) * d;
+#pragma unroll
+          for (int m = 0; m < CPL; ++m)
+            if (lane + TL * m < d) sp[lane + TL * m] = x[m];
+        }
+        ++keep_idx;
+        keep_step += a.thinning;
       }
     }
-    // sample bookkeeping
-    int out = -1;
-    if (step == keep_step) {
-      if (!(scalar && skip)) out = keep_idx;
-      ++keep_idx;
-      keep_step += a.thinning;
-    }
-    if (out >= 0 && out < a.n_rounds && live) {
-      double* sp = a.samples + ((int64_t)out * C + chain) * d;
-      if (h0) sp[i0] = x0;
-      if (h1) sp[i1] = x1;
-    }
+    ucur += ns - __popc(zmask & (SB == 32 ? 0xffffffffu : (1u << (SB & 31)) - 1u));
   }
+  if (injected) cp_async_wait0();
   if (live) {
-    if (h0) a.x[chain * d + i0] = x0;
-    if (h1) a.x[chain * d + i1] = x1;
+#pragma unroll
+    for (int m = 0; m < CPL; ++m)
+      if (lane + TL * m < d) a.x[chain * d + lane + TL * m] = x[m];
     if (lane == 0 && a.status) a.status[chain] = status;
   }
 }
 
-template <int L, int MAXK>
-int launch_har_k(const HarArgs& a, unsigned grid, cudaStream_t s) {
-  const size_t smem = (size_t)(kHarThreads / L) * har_team_stride<L, MAXK>(a.d) * 8;
-  if (cudaFuncSetAttribute(har_kernel<L, MAXK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess) {
+template <int TL, int CPL, int RPL, int SB, int H>
+int launch_har_k(const HarArgs& a, cudaStream_t s) {
+  const HarLayout L = har_layout(a.d, a.cap, SB, a.dirs != nullptr, a.maps != nullptr && a.dirs == nullptr);
+  const size_t smem = (size_t)(kHarThreads / TL) * L.total * 8;
+  auto kern = a.mode == ART_HAR_SCALAR ? har_kernel<TL, CPL, RPL, SB, H, true> : har_kernel<TL, CPL, RPL, SB, H, false>;
+  if (smem > 227 * 1024 ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     cudaGetLastError();
     set_error("art_hit_and_run: cannot reserve %zu bytes of shared memory", smem);
     return ART_E_UNSUPPORTED;
   }
-  cudaFuncSetAttribute(har_kernel<L, MAXK>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                       (int)cudaSharedmemCarveoutMaxShared);
+  cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
   cudaGetLastError();
+  const unsigned grid = (unsigned)((a.n_chains * TL + kHarThreads - 1) / kHarThreads);
   prof_begin("hit_and_run", s);
-  har_kernel<L, MAXK><<<grid, kHarThreads, smem, s>>>(a);
+  kern<<<grid, kHarThreads, smem, s>>>(a);
   prof_end(s);
   count_launch();
   return check_launch("art_hit_and_run");
 }
 
-template <int L>
-int launch_har_l(const HarArgs& a, int maxk, cudaStream_t s) {
-  const int64_t threads = a.n_chains * L;
-  const unsigned grid = (unsigned)((threads + kHarThreads - 1) / kHarThreads);
-  if (maxk <= 4) return launch_har_k<L, 4>(a, grid, s);
-  if (maxk <= 8) return launch_har_k<L, 8>(a, grid, s);
-  if (maxk <= 16) return launch_har_k<L, 16>(a, grid, s);
-  return launch_har_k<L, 32>(a, grid, s);
+// A warp per chain while the device has idle warps for it, else the narrowest
+// team that holds a coordinate and at most four rows a lane.
+template <int H>
+int launch_har_narrow(const HarArgs& a, cudaStream_t s) {  // d <= 8
+  if (a.n_chains <= (int64_t)8 * device_sm_count()) return launch_har_k<32, 1, 1, 32, H>(a, s);
+  if (a.cap <= 8) return launch_har_k<8, 1, 1, 8, H>(a, s);
+  return a.cap <= 16 ? launch_har_k<8, 1, 2, 8, H>(a, s) : launch_har_k<8, 1, 4, 8, H>(a, s);
+}
+int launch_har(const HarArgs& a, cudaStream_t s) {
+  if (a.d <= 2) return launch_har_narrow<1>(a, s);
+  if (a.d <= 4) return launch_har_narrow<2>(a, s);
+  if (a.d <= 8) return launch_har_narrow<4>(a, s);
+  if (a.d <= 16) {
+    if (a.n_chains <= (int64_t)8 * device_sm_count()) return launch_har_k<32, 1, 1, 32, 8>(a, s);
+    return a.cap <= 16 ? launch_har_k<16, 1, 1, 16, 8>(a, s) : launch_har_k<16, 1, 2, 16, 8>(a, s);
+  }
+  if (a.d <= 32) return launch_har_k<32, 1, 1, 32, 16>(a, s);
+  return launch_har_k<32, 2, 1, 16, 32>(a, s);
 }
 
 }  // namespace
@@ -358,13 +547,6 @@ extern "C" int art_hit_and_run(const ArtPolytopes* P, const ArtChains* C, art_st
   a.dirs = C->directions; a.unif = C->uniforms; a.mode = C->mode;
   a.burn_in = C->burn_in; a.thinning = C->thinning; a.n_rounds = C->n_rounds;
   a.counter_base = C->counter_base; a.samples = C->samples; a.status = C->status;
-  cudaStream_t s = (cudaStream_t)stream;
-  const int half = (P->dim + 1) / 2;
-  const int maxk = P->max_rows;
-  if (half <= 1) return launch_har_l<1>(a, maxk, s);
-  if (half <= 2) return launch_har_l<2>(a, maxk, s);
-  if (half <= 4) return launch_har_l<4>(a, maxk, s);
-  if (half <= 8) return launch_har_l<8>(a, maxk, s);
-  if (half <= 16) return launch_har_l<16>(a, maxk, s);
-  return launch_har_l<32>(a, maxk, s);
+  a.cap = P->max_rows <= 4 ? 4 : (P->max_rows <= 8 ? 8 : (P->max_rows <= 16 ? 16 : 32));
+  return launch_har(a, (cudaStream_t)stream);
 }

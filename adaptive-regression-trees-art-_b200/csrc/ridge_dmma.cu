@@ -60,14 +60,6 @@ template <int MAXNB> struct DmLayout {
 };
 constexpr int kQuadStride = 12;  // row stride of the quadratic kinds (d <= 8)
 
-// Asynchronous copies global -> shared of 8 or 16 bytes; `live` off writes zeros.
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, bool live) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(live ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool live) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
-
 __device__ void warp_write_failed(const RidgeArgs& a, int k, int p, int32_t status, double lam,
                                   uint32_t info) {
   const int lane = threadIdx.x & 31;
@@ -244,7 +236,7 @@ __device__ int gram_units(const RidgeArgs& a, const RidgeItem& it, unsigned char
       cp_async8(dst + (uint32_t)(lane * rs + d + 1) * 8u, a.y + it.r0 + r + (live ? lane : 0), live);
       if (a.w) cp_async8(qb + (uint32_t)(h * 32 + lane) * 8u, a.w + it.r0 + r + (live ? lane : 0), live);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    cp_async_commit();
   };
   int bad = 0;
   int unit = u0, h = 0;
@@ -258,8 +250,8 @@ __device__ int gram_units(const RidgeArgs& a, const RidgeItem& it, unsigned char
     const int next_rows = (int)min((int64_t)RS, next_end - rn);
     __syncwarp();  // every lane is done with the other tile
     if (next_rows > 0) issue(rn, next_rows, h ^ 1);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else cp_async_commit();
+    cp_async_wait1();
     const double* xt = X0 + h * T::kTile;
     double* qt = Q0 + h * 32;
     const int rows4 = (rows + 3) & ~3;
@@ -320,7 +312,7 @@ __device__ int gram_units(const RidgeArgs& a, const RidgeItem& it, unsigned char
       unit_end = next_end;
     }
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  cp_async_wait0();
   if (!part && it.n == 0)
     for (int e = lane; e < E; e += 32) G[e] = 0.0;
   __syncwarp();
