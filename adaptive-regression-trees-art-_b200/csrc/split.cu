@@ -28,6 +28,7 @@
 #include "bulk.cuh"
 #include "common.cuh"
 #include "linalg.cuh"
+#include "split.cuh"
 #include "tcgen05.cuh"
 
 namespace art {
@@ -42,9 +43,8 @@ constexpr int kMaxCH = 256;      // rows per chunk: a multiple of 32 up to this
 constexpr int kMaxP = 64;        // child model features
 constexpr int kMaxRg = 16;       // restarts per work item
 constexpr int kRedSlots = 5;     // (restart, component) accumulators per thread
-constexpr int kBuckets = 64;
+constexpr int kBuckets = kSplitBuckets;
 constexpr int kMaxStages = 8;    // row-stage ring depth (chunks in flight)
-constexpr int kErrSlot = 2 + 2 * kBuckets;  // counts[kErrSlot]: a bounded wait gave up
 // Gangs: with at most two restarts per node, a node of n rows is split by
 // min(kGangMax, ceil(n / kGangRows)) CTAs that take interleaved chunks and
 // add their pass sums in rank order through global scratch.  The gang size
@@ -72,53 +72,6 @@ constexpr int kTcAOp = (kTcEntries / 8) * kTcSBO;    // one A array (hi or lo): 
 constexpr int kTcBOp = (32 / 8) * kTcSBO;            // one B array: 4 KB
 constexpr int kTcDrain = 4;
 constexpr uint32_t kTcCols = 64;                     // TMEM columns: two tiles x N <= 32
-
-struct SplitArgs {
-  int64_t K;
-  const int64_t* row_offsets;
-  const int64_t* x_offsets;
-  const int32_t* dims;
-  const int32_t* features;
-  const double* x;
-  const double* y;
-  const double* temperature;
-  const double* ridge;
-  const double* parent_loss;
-  const int8_t* fallback;
-  const double* theta0;
-  int64_t theta0_stride;
-  const uint64_t* node_keys;
-  const int32_t* min_side;  // per-node minimum side count or NULL
-  ArtSplitParams prm;
-  int R, Rg, groups, dmax, pmax, H, TC, S, CH;
-  int mixed;  // ART_PRECISION_MIXED: gates in single precision
-  int tc;     // mixed form with the soft-pass Grams on the tensor cores
-  int dg;     // side Grams as FP64 MMA tiles (8 x 8 blocks of (q psi)^T psi, at most kDgMax per warp)
-  // per (node, restart) results, index k * R + r
-  double* r_theta;   // [.. ][dmax + 1]
-  double* r_loss;
-  double* r_beta;    // [..][2][pmax]
-  double* r_child;   // [..][2]
-  double* r_ridge;   // [..][2]
-  int32_t* r_nright;
-  int32_t* r_iters;
-  int32_t* r_stop;
-  int32_t* r_fail;
-  int32_t* r_flags;
-  int32_t* r_fbiter;
-  double* r_alpha;
-  double* tr_loss;
-  double* tr_step;
-  int32_t* tr_back;
-  double* tr_gnorm;
-  // work queue
-  int32_t* counts;   // [0] entries, [1] cursor, [2..2+64) hist, [66..130) start
-  int4* items;       // queue entries (item, gang rank, gang size, 0)
-  int gang_on, nslots, gang_P;  // gangs enabled; scratch slots; doubles per rank partial
-  int4* gang_rec;    // [K * groups]: slot + 1, barrier arrivals, members done, abort
-  int32_t* slot_flags;  // [nslots]
-  double* gang_scratch; // [nslots][2][kGangMax][gang_P]
-};
 
 // Shared-memory layout for a given (dmax, pmax, Rg, H, S, CH): `ring` holds S
 // stages of CH rows of x and y (bulk copies in flight), `bars` their
@@ -202,33 +155,12 @@ __device__ __forceinline__ double group_sum(double v, int RG) {
   return v;
 }
 
-// D = A B + D for one 8 x 8 x 4 FP64 tile (warp-wide): lane l holds
-// A[l / 4][l % 4], B[l % 4][l / 4] and D[l / 4][2 (l % 4) + {0, 1}].
-__device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-      : "+d"(c[0]), "+d"(c[1])
-      : "d"(a), "d"(b));
-}
-
 struct Item {
   int64_t r0, n, xoff;
   int d, kind, p, pa, E;
   double T0, ridge;
   int k, g, rbase, rn;  // node, group, first restart, restarts in this item
 };
-
-__device__ __forceinline__ double sigm(double s) {
-  s = fmin(fmax(s, -50.0), 50.0);  // objectives.py:49-51
-  return 1.0 / (1.0 + exp(-s));
-}
-
-// Mixed form: the gate in single precision with CUDA's fast exponential
-// (relative error ~1e-7, inside the form's 1e-5 objective tolerance); the
-// score, residuals, solves and every sum stay FP64.
-__device__ __forceinline__ double sigm32(double s) {
-  const float sf = fminf(fmaxf((float)s, -50.0f), 50.0f);
-  return (double)__frcp_rn(1.0f + __expf(-sf));
-}
 
 // Entry e of the packed lower triangle -> (i, j), i >= j.
 __device__ __forceinline__ void entry_ij(int e, int& i, int& j) {
@@ -287,12 +219,18 @@ __device__ __forceinline__ int gang_size(const SplitArgs& a, int64_t n) {
   if (!a.gang_on) return 1;
   return (int)min((int64_t)kGangMax, max((int64_t)1, (n + kGangRows - 1) / kGangRows));
 }
+// Rows a node is ranked by: in the warp form's wide levels, models of more than
+// 23 features always take a gang, so they rank with the smallest of those.
+__device__ __forceinline__ int64_t plan_rows(const SplitArgs& a, int64_t k, int64_t n) {
+  if (a.warp && feature_count(a.dims[k], a.features[k]) + 1 > 24) return max(n, (int64_t)1023);
+  return n;
+}
 __global__ void split_plan_hist(SplitArgs a) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.K * a.groups) return;
   const int64_t k = t / a.groups;
   const int64_t n = a.row_offsets[k + 1] - a.row_offsets[k];
-  const int b = kBuckets - 1 - max(0, min(kBuckets - 1, ilogb((double)(n + 1))));
+  const int b = split_bucket(plan_rows(a, k, n));
   atomicAdd(&a.counts[2 + b], gang_size(a, n));
 }
 __global__ void split_plan_scan(SplitArgs a) {
@@ -310,7 +248,7 @@ __global__ void split_plan_scatter(SplitArgs a) {
   if (t >= a.K * a.groups) return;
   const int64_t k = t / a.groups;
   const int64_t n = a.row_offsets[k + 1] - a.row_offsets[k];
-  const int b = kBuckets - 1 - max(0, min(kBuckets - 1, ilogb((double)(n + 1))));
+  const int b = split_bucket(plan_rows(a, k, n));
   const int G = gang_size(a, n);
   // a gang's members take consecutive entries, so they are popped together
   const int slot = atomicSub(&a.counts[2 + b], G) - G;
@@ -572,7 +510,7 @@ struct SplitCta {
             const int c = code[u] & 0xff, I = (code[u] >> 8) & 0xff, J = code[u] >> 16;
             const double av = in ? Q[row * qs + c] * prow[8 * I] : 0.0;
             const double bv = in ? prow[8 * J] : 0.0;
-            dmma_884(acc[u], av, bv);
+            split_dmma(acc[u], av, bv);
           }
         }
       }
@@ -1542,827 +1480,6 @@ __device__ void SplitCta<TC, TCG>::run(int item_id, int rank, int members) {
   gang_end();
 }
 
-// ============================================ warp-per-restart split kernel
-// One warp per (node, restart) work item, no block barriers: each warp
-// streams its node's rows in tiles of 32, keeps its restart's state in
-// registers (uniform across the warp) and a few shared-memory vectors, and
-// runs its own projected-gradient loop.  The row products run on the FP64
-// tensor path (mma.sync m8n8k4 f64, IEEE FP64 products and sums):
-//   * scores and fitted values: [u, f_L, f_R] = psi [w; beta_L; beta_R]
-//     (x sits in a contiguous block of psi's columns for every feature kind);
-//   * side Grams: G_side += (q_side psi)^T psi, lower-triangular 8 x 8 blocks;
-//   * gradient: g = psi^T c over the x columns.
-// Gates, losses and Armijo tests are per-row lane work added across the warp.
-// The trial step and the next Gram share one pass: the candidate theta_c =
-// project(theta + alpha d) is scored as x . w_c - z_c (the frozen-model
-// evaluation of objectives.py:131-160), its frozen loss taken at the current
-// temperature, and the side Grams at theta_c (at the temperature that
-// follows an accepted step) accumulated on the way, so an accepted step
-// needs no separate Gram pass.  Same objective, stop rules, Armijo steps,
-// AdaptiveAlpha, feasibility tracking, hard partition and refits as the CTA
-// kernel above; the summation order differs.
-
-constexpr int kWTile = 32;                                   // rows per tile
-constexpr int kWMaxPa = 24;                                  // p + 1 (augmented with y)
-constexpr int kWMaxD = 23;                                   // inputs
-constexpr int kWThreads = 128;                               // 4 warps per CTA
-constexpr int kWGangLog = 12;                                // gang items: n + 1 >= 2^12 rows
-constexpr int kWWarps = kWThreads / 32;
-
-// Per-warp shared memory (doubles): psi | cf | sc | tc | th | dn | gr | lf |
-// bl | br | A | fidx | xt; psi's row stride is 8 NB + 1 (NB = the kernel's
-// block count), the rest follow from (dmax, pmax).
-struct WLayout {
-  size_t per_warp, total;
-  int xs, ps;
-};
-__host__ __device__ inline WLayout warp_layout(int dmax, int pmax) {
-  WLayout L;
-  const int pa = pmax + 1, E = pa * (pa + 1) / 2, dt = dmax + 1;
-  L.xs = dmax | 1;
-  L.ps = (8 * ((pa + 7) / 8)) | 1;
-  L.per_warp = (size_t)kWTile * L.ps + 5 * kWTile + 5 * dt + 2 * pmax + E + 2 * pa + pa + kWTile * L.xs;
-  L.total = (size_t)kWWarps * L.per_warp * 8;
-  return L;
-}
-
-// A node of n rows is split by the whole CTA (its warps sharing the tiles)
-// when n + 1 >= 2^kWGangLog: on the plan's size buckets, so every gang item
-// precedes every other item in the work list.
-__device__ __forceinline__ bool warp_gang_item(int64_t n) {
-  return ilogb((double)(n + 1)) >= kWGangLog;
-}
-
-__device__ __forceinline__ double wbcast_sum(double v) {
-  // butterfly sum, then lane 0's value: every lane holds the same bits
-  return __shfl_sync(0xffffffffu, warp_sum(v), 0);
-}
-
-// first psi column holding x_1 for each feature kind (x is contiguous there)
-__device__ __forceinline__ int x_column(int kind) {
-  return (kind == ART_FEATURES_POLY1 || kind == ART_FEATURES_POLY2) ? 1 : 0;
-}
-
-// NB 8-column blocks of psi (pa <= 8 NB); the score MMAs take NK = 2 NB
-// 4-column steps.  Fixed trip counts: padding columns and rows are zeros.
-template <int NB>
-struct SplitWarp {
-  static constexpr int NK = 2 * NB;
-  const SplitArgs& a;
-  static constexpr int ps = 8 * NB + 1;  // psi row stride (odd, in doubles)
-  double* base;                          // this warp's shared-memory region
-  bool aff = false;                      // affine features: x is psi's first d columns
-  int lane;
-  // region pointers, recomputed from the launch's (dmax, pmax) where used
-  __device__ double* psi() const { return base; }
-  __device__ double* cf() const { return base + kWTile * ps; }
-  __device__ double* sc() const { return base + kWTile * ps + 2 * kWTile; }
-  __device__ double* tc() const { return base + kWTile * ps + 5 * kWTile; }
-  __device__ double* th() const { return tc() + (a.dmax + 1); }
-  __device__ double* dn() const { return tc() + 2 * (a.dmax + 1); }
-  __device__ double* gr() const { return tc() + 3 * (a.dmax + 1); }
-  __device__ double* lf() const { return tc() + 4 * (a.dmax + 1); }
-  __device__ double* bl() const { return tc() + 5 * (a.dmax + 1); }
-  __device__ double* br() const { return bl() + a.pmax; }
-  __device__ double* A() const { return bl() + 2 * a.pmax; }
-  __device__ int16_t* fidx() const {
-    return (int16_t*)(A() + (a.pmax + 1) * (a.pmax + 2) / 2 + 2 * (a.pmax + 1));
-  }
-  // the x tile: its own buffer, or for affine features psi itself
-  __device__ double* xt() const {
-    return aff ? base : (double*)fidx() + (a.pmax + 1);
-  }  __device__ int xs() const { return aff ? ps : (a.dmax | 1); }
-  __device__ int kq() const { return lane & 3; }   // fragment coordinates of this lane
-  __device__ int mq() const { return lane >> 2; }
-  // item
-  int64_t k, r0, n, xoff, kr;
-  int d, kind, p, pa, E, xcol;
-  int tail, nks, nbx;  // columns of the last block row; score steps and gradient blocks holding data
-  bool narrow;         // tail <= 4: the tail rows of both sides in one MMA per block column
-  double ridge, T0;
-  // restart state (uniform)
-  double loss = 0, dd = 0, tol = 0, gnorm = 0, T = 0, invT = 0, alpha = 0, lamL = 0, lamR = 0;
-  double hlossL = 0, hlossR = 0;
-  int nright = 0, iters = 0, stop = 0, fail = 0, feasit = -1;
-  bool active = false, hasfeas = false, conv = false, fbk = false;
-
-  // gang: the CTA's warps share one large item, warp grank taking tiles
-  // grank, grank + gsize, ...; every pass ends with the partial sums of all
-  // members added in member order, so each member holds the same totals and
-  // runs the same control flow
-  int grank = 0, gsize = 1;
-  size_t pw;  // doubles per warp region
-
-  __device__ SplitWarp(const SplitArgs& a_, unsigned char* sm, int warp) : a(a_) {
-    pw = warp_layout(a.dmax, a.pmax).per_warp;
-    base = (double*)sm + (size_t)warp * pw;
-    lane = threadIdx.x & 31;
-  }
-  __device__ int64_t tile0() const { return (int64_t)grank * kWTile; }
-  __device__ int64_t tstep() const { return (int64_t)gsize * kWTile; }
-  __device__ void gang_bar() const { asm volatile("bar.sync 1, %0;" ::"r"(kWThreads) : "memory"); }
-  // Gang sums of per-lane partials: each member stores its partials in
-  // slots of its psi region (free between passes), a barrier, then every
-  // member adds slot c of all members in member order (gang_end restores
-  // psi's zero padding after the second barrier).
-  __device__ void gput(int c, double v) const { base[c * kWTile + lane] = v; }
-  __device__ double gsum(int c) const {
-    const double* b0 = base - (size_t)grank * pw;
-    double t = b0[c * kWTile + lane];
-    for (int g = 1; g < gsize; ++g) t += b0[(size_t)g * pw + c * kWTile + lane];
-    return t;
-  }
-  __device__ void gang_end() {
-    gang_bar();
-    for (int f = pa; f < ps; ++f) base[lane * ps + f] = 0.0;
-    __syncwarp();
-  }
-
-  // Tile rows [t0, t0 + rows): x (coalesced copy) and psi = [phi(x); y],
-  // rows past the end zero.  Returns the row count; ends with __syncwarp.
-  __device__ int load_tile(int64_t t0, double& yv) {
-    const int rows = (int)min((int64_t)kWTile, n - t0);
-    const double* src = a.x + xoff + t0 * d;
-    const int tot = rows * d;
-    const uint32_t inv = 65536u / (uint32_t)d + 1u;  // e / d by a multiply (e < 32 * 23)
-    double* xd = xt();
-    const int xsv = xs();
-    __syncwarp();
-    for (int e = lane; e < tot; e += 32) {
-      const int rr = (int)(((uint32_t)e * inv) >> 16), i = e - rr * d;
-      xd[rr * xsv + i] = __ldg(src + e);
-    }
-    yv = lane < rows ? __ldg(a.y + r0 + t0 + lane) : 0.0;
-    __syncwarp();
-    double* pr = psi() + lane * ps;
-    const double* xr = xt() + lane * xs();
-    if (aff && lane < rows) {
-      pr[d] = 1.0;
-      pr[p] = yv;
-    } else if (lane < rows) {
-      for (int f = 0; f < p; ++f) {
-        const int ia = fidx()[2 * f], ib = fidx()[2 * f + 1];
-        pr[f] = (ia < 0 ? 1.0 : xr[ia]) * (ib < 0 ? 1.0 : xr[ib]);
-      }
-      pr[p] = yv;
-    } else {
-      for (int f = 0; f <= p; ++f) pr[f] = 0.0;
-    }
-    __syncwarp();
-    return rows;
-  }
-
-  // B fragments of [w; beta_L; beta_R] (columns 0, 1, 2; rows = psi columns)
-  // for the score MMAs: lane (k, m) holds B[4 s + k][m] of step s.
-  __device__ void score_operand(const double* w, double (&b)[NK]) const {
-#pragma unroll
-    for (int s = 0; s < NK; ++s) {
-      const int f = 4 * s + kq();
-      double v = 0.0;
-      if (mq() == 0) v = (f >= xcol && f < xcol + d) ? w[f - xcol] : 0.0;
-      else if (mq() == 1) v = f < p ? bl()[f] : 0.0;
-      else if (mq() == 2) v = f < p ? br()[f] : 0.0;
-      b[s] = v;
-    }
-  }
-
-  // u, f_L, f_R of this lane's row: psi [w; beta_L; beta_R] by MMAs over
-  // 8-row blocks, staged through shared memory.  Call after load_tile.
-  __device__ void scores(const double (&b)[NK], double& u, double& fl, double& fr) {
-#pragma unroll
-    for (int rb = 0; rb < 4; ++rb) {
-      double c[2] = {0.0, 0.0};
-      const double* pr = psi() + (8 * rb + mq()) * ps + kq();
-#pragma unroll
-      for (int s = 0; s < NK; ++s)
-        if (s < NK - 1 || nks == NK) dmma_884(c, pr[4 * s], b[s]);  // the last step may be all padding
-      if (kq() == 0) { sc()[8 * rb + mq()] = c[0]; sc()[kWTile + 8 * rb + mq()] = c[1]; }
-      else if (kq() == 1) sc()[2 * kWTile + 8 * rb + mq()] = c[0];
-    }
-    __syncwarp();
-    u = sc()[lane];
-    fl = sc()[kWTile + lane];
-    fr = sc()[2 * kWTile + lane];
-    __syncwarp();
-  }
-
-  // G_side += (q_side psi)^T psi over the tile (lower 8 x 8 blocks), the
-  // weights staged in cf.  Rows past the tile's end are zero rows.
-  static constexpr int NBLK = NB * (NB + 1) / 2;  // lower-triangular 8 x 8 blocks
-  //
-  // Narrow tail (the item's last block row holds tail <= 4 columns, or none):
-  // the blocks of the first NB - 1 block rows as above, then the tail rows of
-  // both sides in one MMA per block column: A = psi block J, B = [q_L psi_T,
-  // q_R psi_T] (columns n < tail: left side, tail <= n < 2 tail: right), so
-  // D[m][n] = G_side[T + n'][8 J + m] with T = 8 (NB - 1).  The results sit in
-  // cL's last block row; cR's stays zero.
-  __device__ void gram_tile(double qL, double qR, double (&cL)[NBLK][2], double (&cR)[NBLK][2]) {
-    cf()[lane] = qL;
-    cf()[kWTile + lane] = qR;
-    __syncwarp();
-    if (narrow) {
-      constexpr int T = 8 * (NB - 1);
-      const int tcol = mq() < tail ? mq() : mq() - tail;
-      const bool tl = tail > 0 && mq() < 2 * tail;
-#pragma unroll 2
-      for (int k0 = 0; k0 < kWTile; k0 += 4) {
-        const int row = k0 + kq();
-        const double* pr = psi() + row * ps + mq();
-        const double ql = cf()[row], qr = cf()[kWTile + row];
-        double v[NB];
-#pragma unroll
-        for (int I = 0; I < NB; ++I) v[I] = pr[8 * I];
-#pragma unroll
-        for (int I = 0; I < NB - 1; ++I) {
-          const double aL = ql * v[I], aR = qr * v[I];
-#pragma unroll
-          for (int J = 0; J <= I; ++J) {
-            dmma_884(cL[I * (I + 1) / 2 + J], aL, v[J]);
-            dmma_884(cR[I * (I + 1) / 2 + J], aR, v[J]);
-          }
-        }
-        if (tail > 0) {  // warp-uniform
-          const double bt = tl ? (mq() < tail ? ql : qr) * psi()[row * ps + T + tcol] : 0.0;
-#pragma unroll
-          for (int J = 0; J < NB; ++J) dmma_884(cL[(NB - 1) * NB / 2 + J], v[J], bt);
-        }
-      }
-      __syncwarp();
-      return;
-    }
-#pragma unroll 2
-    for (int k0 = 0; k0 < kWTile; k0 += 4) {
-      const int row = k0 + kq();
-      const double* pr = psi() + row * ps + mq();
-      const double ql = cf()[row], qr = cf()[kWTile + row];
-      double v[NB];
-#pragma unroll
-      for (int I = 0; I < NB; ++I) v[I] = pr[8 * I];
-#pragma unroll
-      for (int I = 0; I < NB; ++I) {
-        const double aL = ql * v[I], aR = qr * v[I];
-#pragma unroll
-        for (int J = 0; J <= I; ++J) {
-          dmma_884(cL[I * (I + 1) / 2 + J], aL, v[J]);
-          dmma_884(cR[I * (I + 1) / 2 + J], aR, v[J]);
-        }
-      }
-    }
-    __syncwarp();
-  }
-
-  // g += psi^T c over the tile (column 0 of the MMA output; c staged in cf).
-  __device__ void grad_tile(double c, double (&g)[NB][2]) {
-    cf()[lane] = c;
-    __syncwarp();
-#pragma unroll
-    for (int k0 = 0; k0 < kWTile; k0 += 4) {
-      const int row = k0 + kq();
-      const double* pr = psi() + row * ps + mq();
-      const double b = mq() == 0 ? cf()[row] : 0.0;
-#pragma unroll
-      for (int I = 0; I < NB; ++I)
-        if (I < NB - 1 || nbx == NB) dmma_884(g[I], pr[8 * I], b);  // blocks holding x columns
-    }
-    __syncwarp();
-  }
-
-  __device__ double gate(double s) const { return a.mixed ? sigm32(s) : sigm(s); }
-
-  __device__ void run(int item);
-  // the side Gram blocks (and one extra per-lane partial) summed over the gang
-  __device__ void gang_gram(double (&cL)[NBLK][2], double (&cR)[NBLK][2], double* extra = nullptr) {
-    static_assert(4 * NBLK + 1 <= ps, "gang slots: 32 x ps doubles of psi");
-    if (gsize == 1) return;
-#pragma unroll
-    for (int q = 0; q < NBLK; ++q) {
-      gput(4 * q, cL[q][0]); gput(4 * q + 1, cL[q][1]); gput(4 * q + 2, cR[q][0]); gput(4 * q + 3, cR[q][1]);
-    }
-    if (extra) gput(4 * NBLK, *extra);
-    gang_bar();
-#pragma unroll
-    for (int q = 0; q < NBLK; ++q) {
-      cL[q][0] = gsum(4 * q); cL[q][1] = gsum(4 * q + 1); cR[q][0] = gsum(4 * q + 2); cR[q][1] = gsum(4 * q + 3);
-    }
-    if (extra) *extra = gsum(4 * NBLK);
-    gang_end();
-  }
-  __device__ bool solve_sides(const double (&cL)[NBLK][2], const double (&cR)[NBLK][2]);
-  __device__ void gram_pass(const double* w, bool hard, int req, bool accumulate, double (&cL)[NBLK][2],
-                            double (&cR)[NBLK][2]);
-  __device__ void resid_pass();
-  __device__ double trial_gram_pass(double invT_next, double (&cL)[NBLK][2], double (&cR)[NBLK][2]);
-  __device__ void hard_losses();
-};
-
-// Both sides' ridge solves from the accumulated Gram blocks; false (restart
-// failed) when either factorisation fails.
-template <int NB>
-__device__ bool SplitWarp<NB>::solve_sides(const double (&cL)[NBLK][2], const double (&cR)[NBLK][2]) {
-  double* z_ = A() + E;
-  bool ok = true;
-  for (int side = 0; side < 2; ++side) {
-    __syncwarp();
-#pragma unroll
-    for (int I = 0; I < NB; ++I)
-#pragma unroll
-      for (int J = 0; J <= I; ++J)
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const int i = 8 * I + mq(), j = 8 * J + 2 * kq() + t;
-          if ((!narrow || I < NB - 1) && i < pa && j <= i)
-            A()[i * (i + 1) / 2 + j] = side ? cR[I * (I + 1) / 2 + J][t] : cL[I * (I + 1) / 2 + J][t];
-        }
-    if (narrow && tail > 0) {
-      // tail rows: lane (m, k) holds D[m][n], n = 2 k + t: side n / tail, row
-      // T + n % tail, column 8 J + m
-#pragma unroll
-      for (int J = 0; J < NB; ++J)
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const int n_ = 2 * kq() + t;
-          if (n_ < 2 * tail && (n_ >= tail) == (side == 1)) {
-            const int i = 8 * (NB - 1) + (n_ < tail ? n_ : n_ - tail), j = 8 * J + mq();
-            if (i < pa && j <= i) A()[i * (i + 1) / 2 + j] = cL[(NB - 1) * NB / 2 + J][t];
-          }
-        }
-    }
-    __syncwarp();
-    double lam;
-    if (warp_ridge_solve(A(), z_, p, ridge, lam)) {
-      ok = false;
-      continue;
-    }
-    double* beta = side ? br() : bl();
-    for (int i = lane; i < p; i += 32) beta[i] = z_[i];
-    if (side) lamR = lam; else lamL = lam;
-  }
-  __syncwarp();
-  return ok;
-}
-
-// Side Grams at theta = (w, w[d]) over all rows.  Soft: gates with the
-// weight floor; hard: exact sides (weights 1 / 0) and the right-side count,
-// the Gram skipped when a side is below req or `accumulate` is off.
-template <int NB>
-__device__ void SplitWarp<NB>::gram_pass(const double* w, bool hard, int req, bool accumulate,
-                                         double (&cL)[NBLK][2], double (&cR)[NBLK][2]) {
-  const double z = w[d];
-  double b[NK];
-  score_operand(w, b);
-#pragma unroll
-  for (int q = 0; q < NBLK; ++q) cL[q][0] = cL[q][1] = cR[q][0] = cR[q][1] = 0.0;
-  int cnt = 0;
-  if (hard) {  // count first: the Grams are needed only when both sides are large enough
-    for (int64_t t0 = tile0(); t0 < n; t0 += tstep()) {
-      double yv;
-      const int rows = load_tile(t0, yv);
-      if (lane < rows) cnt += right_side(psi() + lane * ps + xcol, w, d, z) ? 1 : 0;
-    }
-    if (gsize > 1) {  // integers: exact in any order
-      gput(0, (double)cnt);
-      gang_bar();
-      cnt = (int)gsum(0);
-      gang_end();
-    }
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    nright = cnt;
-    if (nright < req || (int)n - nright < req || !accumulate) return;
-  }
-  for (int64_t t0 = tile0(); t0 < n; t0 += tstep()) {
-    double yv;
-    const int rows = load_tile(t0, yv);
-    double qL = 0.0, qR = 0.0;
-    if (hard) {
-      if (lane < rows) {
-        const bool right = right_side(psi() + lane * ps + xcol, w, d, z);
-        qL = right ? 0.0 : 1.0;
-        qR = right ? 1.0 : 0.0;
-      }
-    } else {
-      double u, fl, fr;
-      scores(b, u, fl, fr);
-      if (lane < rows) {
-        const double pi = gate((u - z) * invT);
-        qL = fmax(1.0 - pi, a.prm.weight_floor);
-        qR = fmax(pi, a.prm.weight_floor);
-      }
-    }
-    gram_tile(qL, qR, cL, cR);
-  }
-  gang_gram(cL, cR);
-}
-
-// Soft residual pass at theta with the current child models: loss,
-// gradient, n_right (pi >= 0.5), then the projected gradient, its norm and
-// the directional derivative.
-template <int NB>
-__device__ void SplitWarp<NB>::resid_pass() {
-  const double z = th()[d];
-  const double inv_n = 1.0 / (double)n;
-  double b[NK];
-  score_operand(th(), b);
-  double g[NB][2];
-#pragma unroll
-  for (int I = 0; I < NB; ++I) g[I][0] = g[I][1] = 0.0;
-  double sl = 0.0, sa = 0.0, snr = 0.0;
-  for (int64_t t0 = tile0(); t0 < n; t0 += tstep()) {
-    double yv;
-    const int rows = load_tile(t0, yv);
-    double u, fl, fr;
-    scores(b, u, fl, fr);
-    double c = 0.0;
-    if (lane < rows) {
-      const double pi = gate((u - z) * invT);
-      const double eL = yv - fl, eR = yv - fr;
-      const double eL2 = eL * eL, eR2 = eR * eR;
-      c = (eR2 - eL2) * pi * (1.0 - pi) * inv_n;
-      sl += (1.0 - pi) * eL2 + pi * eR2;
-      sa += c;
-      snr += pi >= 0.5 ? 1.0 : 0.0;
-    }
-    grad_tile(c, g);
-  }
-  if (gsize > 1) {
-#pragma unroll
-    for (int I = 0; I < NB; ++I) gput(I, g[I][0]);  // column 0 only is used
-    gput(NB, sl); gput(NB + 1, sa); gput(NB + 2, snr);
-    gang_bar();
-#pragma unroll
-    for (int I = 0; I < NB; ++I) g[I][0] = gsum(I);
-    sl = gsum(NB); sa = gsum(NB + 1); snr = gsum(NB + 2);
-    gang_end();
-  }
-  // psi column 8 I + m of the gradient sits in lane (k = 0, m), block I
-  __syncwarp();
-  if (kq() == 0) {
-#pragma unroll
-    for (int I = 0; I < NB; ++I) {
-      const int col = 8 * I + mq() - xcol;
-      if (col >= 0 && col < d) gr()[col] = g[I][0] / T;
-    }
-  }
-  const double tot_l = wbcast_sum(sl), tot_a = wbcast_sum(sa), tot_nr = wbcast_sum(snr);
-  if (lane == 0) gr()[d] = -tot_a / T;
-  __syncwarp();
-  loss = tot_l / (double)n;
-  nright = (int)tot_nr;
-  // projected gradient and its norm (splitters.py:86-98), evaluated by every
-  // lane in the same order
-  const double* w = th();
-  double gw = 0.0, nrm2 = 0.0;
-  for (int i = 0; i < d; ++i) gw += gr()[i] * w[i];
-  for (int i = 0; i < d; ++i) {
-    const double pg = gr()[i] - gw * w[i];
-    nrm2 += pg * pg;
-  }
-  nrm2 += gr()[d] * gr()[d];
-  __syncwarp();
-  if (lane == 0) {
-    for (int i = 0; i < d; ++i) dn()[i] = -(gr()[i] - gw * w[i]);
-    dn()[d] = -gr()[d];
-  }
-  __syncwarp();
-  gnorm = sqrt(nrm2);
-  double s = 0.0;
-  for (int i = 0; i <= d; ++i) s += gr()[i] * dn()[i];
-  dd = s;
-}
-
-// One Armijo candidate theta_c (in tc): its frozen-model loss at the current
-// temperature (objectives.py:145-156), and the side Grams at theta_c with the
-// gates at invT_next, the temperature that follows an accepted step.
-template <int NB>
-__device__ double SplitWarp<NB>::trial_gram_pass(double invT_next, double (&cL)[NBLK][2], double (&cR)[NBLK][2]) {
-  const double z = tc()[d];
-  double b[NK];
-  score_operand(tc(), b);
-#pragma unroll
-  for (int q = 0; q < NBLK; ++q) cL[q][0] = cL[q][1] = cR[q][0] = cR[q][1] = 0.0;
-  const bool same_t = invT_next == invT;
-  double sl = 0.0;
-  for (int64_t t0 = tile0(); t0 < n; t0 += tstep()) {
-    double yv;
-    const int rows = load_tile(t0, yv);
-    double u, fl, fr;
-    scores(b, u, fl, fr);
-    double qL = 0.0, qR = 0.0;
-    if (lane < rows) {
-      const double pi = gate((u - z) * invT);
-      const double eL = yv - fl, eR = yv - fr;
-      sl += (1.0 - pi) * (eL * eL) + pi * (eR * eR);
-      const double pn = same_t ? pi : gate((u - z) * invT_next);
-      qL = fmax(1.0 - pn, a.prm.weight_floor);
-      qR = fmax(pn, a.prm.weight_floor);
-    }
-    gram_tile(qL, qR, cL, cR);
-  }
-  gang_gram(cL, cR, &sl);
-  return wbcast_sum(sl) / (double)n;
-}
-
-// Hard losses: mean squared residual of each side's hard model.
-template <int NB>
-__device__ void SplitWarp<NB>::hard_losses() {
-  const double z = th()[d];
-  double b[NK];
-  score_operand(th(), b);
-  double sL = 0.0, sR = 0.0;
-  for (int64_t t0 = tile0(); t0 < n; t0 += tstep()) {
-    double yv;
-    const int rows = load_tile(t0, yv);
-    double u, fl, fr;
-    scores(b, u, fl, fr);
-    if (lane < rows) {
-      const bool right = right_side(psi() + lane * ps + xcol, th(), d, z);
-      const double e = yv - (right ? fr : fl);
-      (right ? sR : sL) += e * e;
-    }
-  }
-  if (gsize > 1) {
-    gput(0, sL); gput(1, sR);
-    gang_bar();
-    sL = gsum(0); sR = gsum(1);
-    gang_end();
-  }
-  const double tl = wbcast_sum(sL), trr = wbcast_sum(sR);
-  const int nl = (int)n - nright;
-  hlossL = tl / nl;
-  hlossR = trr / nright;
-  loss = (double)nl / n * hlossL + (double)nright / n * hlossR;
-}
-
-template <int NB>
-__device__ void SplitWarp<NB>::run(int item) {
-  const ArtSplitParams& P = a.prm;
-  k = item / a.R;
-  kr = (int64_t)item;  // items are k * R + restart
-  r0 = a.row_offsets[k];
-  n = a.row_offsets[k + 1] - r0;
-  xoff = a.x_offsets[k];
-  d = a.dims[k];
-  kind = a.features[k];
-  p = feature_count(d, kind);
-  pa = p + 1;
-  E = pa * (pa + 1) / 2;
-  xcol = x_column(kind);
-  tail = pa - 8 * (NB - 1);
-  narrow = tail <= 4;
-  nks = (p + 3) >> 2;
-  nbx = (xcol + d + 7) >> 3;
-  T0 = a.temperature[k];
-  ridge = a.ridge[k];
-  const int req = max(a.min_side ? max(1, a.min_side[k]) : P.min_side_points,
-                      (int)ceil(P.min_side_fraction * (double)n));
-  const bool fb_allowed = a.fallback ? a.fallback[k] != 0 : false;
-  const int M = P.max_iters;
-  aff = kind == ART_FEATURES_AFFINE;
-  __syncwarp();
-  for (int i = lane; i < kWTile * ps; i += 32) psi()[i] = 0.0;  // columns past pa stay zero
-  for (int f = lane; f < p; f += 32) {
-    int ia, ib;
-    feature_factors(d, kind, f, ia, ib);
-    fidx()[2 * f] = (int16_t)ia;
-    fidx()[2 * f + 1] = (int16_t)ib;
-  }
-  // initial theta: projected theta0 (splitters.py:379)
-  const double* t0 = a.theta0 + kr * a.theta0_stride;
-  double nrm2 = 0.0;
-  for (int i = 0; i < d; ++i) nrm2 += t0[i] * t0[i];
-  const double nrm = sqrt(nrm2);
-  active = true;
-  fail = 0;
-  if (!(nrm > 1e-12) || !isfinite(nrm)) { active = false; fail = ART_SPLIT_INVALID; }
-  for (int i = lane; i < d; i += 32) th()[i] = t0[i] / nrm;
-  if (lane == 0) th()[d] = t0[d];
-  __syncwarp();
-  T = T0;
-  invT = 1.0 / T0;
-  alpha = fmin(fmax(P.alpha0, P.alpha_min), P.alpha_max);
-  stop = ART_STOP_MAX_ITERS;
-  feasit = -1;
-  hasfeas = conv = fbk = false;
-  iters = 0;
-  nright = 0;
-  loss = gnorm = dd = 0.0;
-  lamL = lamR = 0.0;
-  if (n == 0) { active = false; fail = ART_SPLIT_MIN_SIDE_POINTS; }
-  auto record_trace = [&](int iter) {
-    if (lane != 0 || grank != 0) return;
-    if (a.tr_loss) a.tr_loss[kr * (M + 1) + iter] = loss;
-    if (a.tr_gnorm) a.tr_gnorm[kr * (M + 1) + iter] = gnorm;
-  };
-  auto save_feasible = [&](int it_) {
-    if (min(nright, (int)n - nright) >= req) {
-      hasfeas = true;
-      feasit = it_;
-      __syncwarp();
-      for (int i = lane; i <= d; i += 32) lf()[i] = th()[i];
-      __syncwarp();
-    }
-  };
-  double cL[NBLK][2], cR[NBLK][2];
-  // evaluate(theta): child fits from the Grams, then the residual pass
-  auto fit_and_resid = [&]() {
-    if (!solve_sides(cL, cR)) {
-      active = false;
-      fail = ART_SPLIT_CHOLESKY_FAILURE;
-      return;
-    }
-    resid_pass();
-  };
-  if (active) {
-    gram_pass(th(), false, 0, true, cL, cR);
-    fit_and_resid();
-    if (active) {
-      tol = P.grad_atol + P.grad_rtol * gnorm;
-      save_feasible(0);
-      record_trace(0);
-    }
-  }
-  for (int iter = 0; iter < M && active; ++iter) {
-    // stop checks (splitters.py:424-437)
-    if (gnorm <= tol) { conv = true; stop = ART_STOP_GRADIENT_TOLERANCE; active = false; break; }
-    if (dd >= 0.0) { stop = ART_STOP_NON_DESCENT; active = false; break; }
-    // temperature after an accepted step (the candidate Grams are taken at it)
-    double T_next = T, invT_next = invT;
-    if (P.anneal_ratio != 1.0 && P.max_iters > 1) {
-      T_next = T0 * pow(P.anneal_ratio, (double)(iter + 1) / (double)(P.max_iters - 1));
-      invT_next = 1.0 / T_next;
-    }
-    // Armijo backtracking, one candidate per pass (optimizers.py:72-121),
-    // restarted from the adapted step after a failed attempt
-    bool accept = false;
-    int failures = 0, nb_ = 0;
-    double a_ = P.adaptive_alpha ? alpha : P.alpha0, step = 0.0;
-    const int max_trials = (P.max_backtracks + 1) * P.max_line_search_failures;
-    for (int trial = 0; trial < max_trials; ++trial) {
-      // candidate theta_c = project(theta + alpha d) (splitters.py:451, 497)
-      __syncwarp();
-      if (lane == 0) {
-        double s2 = 0.0;
-        for (int i = 0; i < d; ++i) {
-          const double v = th()[i] + a_ * dn()[i];
-          s2 += v * v;
-        }
-        const double nw = sqrt(s2);
-        for (int i = 0; i < d; ++i) tc()[i] = (th()[i] + a_ * dn()[i]) / nw;
-        tc()[d] = th()[d] + a_ * dn()[d];
-      }
-      __syncwarp();
-      const double fv = trial_gram_pass(invT_next, cL, cR);
-      const double rhs = __dadd_rn(loss, __dmul_rn(__dmul_rn(P.armijo_c, a_), dd));
-      if (fv <= rhs) {
-        accept = true;
-        step = a_;
-        if (P.adaptive_alpha) {  // AdaptiveAlpha.update (optimizers.py:49-66)
-          double na;
-          if (nb_ == 0) na = step * P.alpha_grow;
-          else if (nb_ >= P.heavy_backtrack_threshold) na = step * P.alpha_recovery;
-          else na = step / P.rho;
-          alpha = fmin(fmax(na, P.alpha_min), P.alpha_max);
-        }
-        break;
-      }
-      if (nb_ < P.max_backtracks) {  // next backtrack
-        ++nb_;
-        a_ *= P.rho;
-        continue;
-      }
-      // attempt failed: the last step tried
-      if (P.adaptive_alpha) alpha = fmin(fmax(a_ * P.rho, P.alpha_min), P.alpha_max);
-      ++failures;
-      int st = -1;
-      if (!P.adaptive_alpha) st = ART_STOP_LINE_SEARCH_FAILED;
-      else if (failures >= P.max_line_search_failures) st = ART_STOP_MAX_LINE_SEARCH_FAILURES;
-      else if (alpha <= P.alpha_min) st = ART_STOP_ALPHA_MIN_REACHED;
-      if (st >= 0) {
-        stop = st;
-        break;
-      }
-      nb_ = 0;
-      a_ = alpha;
-    }
-    if (!accept) {
-      if (stop == ART_STOP_MAX_ITERS) stop = ART_STOP_MAX_LINE_SEARCH_FAILURES;
-      active = false;
-      break;
-    }
-    // commit theta <- theta_c, then the new temperature
-    __syncwarp();
-    for (int i = lane; i <= d; i += 32) th()[i] = tc()[i];
-    __syncwarp();
-    T = T_next;
-    invT = invT_next;
-    iters = iter + 1;
-    if (lane == 0 && grank == 0) {
-      if (a.tr_step) a.tr_step[kr * P.max_iters + iter] = step;
-      if (a.tr_back) a.tr_back[kr * P.max_iters + iter] = nb_;
-    }
-    fit_and_resid();
-    if (active) {
-      save_feasible(iter + 1);
-      record_trace(iter + 1);
-    }
-  }
-  // ------------------------------------------------ finish (splitters.py:584-601)
-  if (fail == 0) {
-    const bool final_ok = min(nright, (int)n - nright) >= req;
-    __syncwarp();
-    if (!final_ok && fb_allowed && hasfeas) {
-      for (int i = lane; i <= d; i += 32) th()[i] = lf()[i];
-      fbk = true;
-    }
-    __syncwarp();
-    double s2 = 0.0;
-    for (int i = 0; i < d; ++i) s2 += th()[i] * th()[i];
-    const double nw = sqrt(s2);
-    __syncwarp();
-    if (lane == 0)
-      for (int i = 0; i < d; ++i) th()[i] = th()[i] / nw;
-    __syncwarp();
-    // hard partition: exact sides and right count; hard child fits when asked
-    gram_pass(th(), true, req, P.hard_refit != 0, cL, cR);
-    if (nright < req || (int)n - nright < req) {
-      fail = ART_SPLIT_MIN_SIDE_POINTS;
-    } else if (P.hard_refit) {
-      if (!solve_sides(cL, cR)) fail = ART_SPLIT_CHOLESKY_FAILURE;
-      else hard_losses();
-    }
-  }
-  // ----------------------------------------------------------- write results
-  __syncwarp();
-  if (lane == 0 && grank == 0) {
-    const int dts = a.dmax + 1;
-    for (int i = 0; i <= d; ++i) a.r_theta[kr * dts + i] = th()[i];
-    a.r_fail[kr] = fail;
-    a.r_stop[kr] = stop;
-    a.r_iters[kr] = iters;
-    a.r_nright[kr] = nright;
-    a.r_flags[kr] = (conv ? 1 : 0) | (fbk ? 2 : 0);
-    a.r_fbiter[kr] = feasit;
-    a.r_alpha[kr] = P.adaptive_alpha ? alpha : P.alpha0;
-    const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    const bool have = P.hard_refit && fail == 0;
-    a.r_loss[kr] = have ? loss : nan;
-    a.r_child[kr * 2] = P.hard_refit ? hlossL : nan;
-    a.r_child[kr * 2 + 1] = P.hard_refit ? hlossR : nan;
-    a.r_ridge[kr * 2] = lamL;
-    a.r_ridge[kr * 2 + 1] = lamR;
-    for (int f = 0; f < p; ++f) {
-      a.r_beta[(kr * 2) * a.pmax + f] = have ? bl()[f] : nan;
-      a.r_beta[(kr * 2 + 1) * a.pmax + f] = have ? br()[f] : nan;
-    }
-  }
-  __syncwarp();
-}
-
-// Resident 4-warp CTAs per SM: 4 (16 warps, a 128-register cap) for up to
-// two blocks; 3 (12 warps, 168 registers) for three, whose six Gram blocks
-// per side would spill under the tighter cap.
-template <int NB>
-__global__ void __launch_bounds__(kWThreads, NB == 3 ? 3 : 4) split_warp_kernel(SplitArgs a) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int s_q;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  SplitWarp<NB> W(a, smem, warp);
-  const int count = a.counts[0];
-  // Items come largest first.  While they are large the whole CTA takes one
-  // at a time (a gang of all its warps); from the first small item on, each
-  // warp pops its own, warp 0 starting with the CTA's last pop.  (One call
-  // site of run keeps it inlined and the state in registers.)
-  bool cta_phase = true;
-  for (;;) {
-    int item = -1;
-    if (cta_phase) {
-      if (threadIdx.x == 0) s_q = atomicAdd(&a.counts[1], 1);
-      __syncthreads();
-      const int q = s_q;
-      __syncthreads();
-      if (q >= count) return;
-      item = a.items[q].x;
-      const int64_t k = item / a.R;
-      if (warp_gang_item(a.row_offsets[k + 1] - a.row_offsets[k])) {
-        W.grank = warp;
-        W.gsize = kWWarps;
-      } else {
-        cta_phase = false;
-        W.grank = 0;
-        W.gsize = 1;
-        if (warp != 0) item = -1;
-      }
-    }
-    if (item < 0) {
-      int q = 0;
-      if (lane == 0) q = atomicAdd(&a.counts[1], 1);
-      q = __shfl_sync(0xffffffffu, q, 0);
-      if (q >= count) return;
-      item = a.items[q].x;
-    }
-    W.run(item);
-  }
-}
-
 // MINB resident CTAs per SM: 1 keeps every register a thread wants and the
 // deepest row ring; 2 doubles the warps that hide the per-row latency of the
 // passes at the cost of a 128-register cap and half the shared memory
@@ -2702,10 +1819,10 @@ extern "C" int art_split_level(const ArtSplitProblem* pr, const ArtSplitParams* 
       }
     }
   }
-  // Warp-per-restart form: asked for, the level fits its register tiles and
-  // no tensor-core Gram is in use
-  const bool use_warp = prm->restart_warps == 1 && !use_tc && pr->max_dim <= kWMaxD &&
-                        pr->max_features + 1 <= kWMaxPa;
+  // Warp form: asked for, or with at most two restarts a node (nothing to
+  // share then between the restarts of a CTA), where the level fits its
+  // register tiles and no tensor-core Gram is in use
+  const bool use_warp = (prm->restart_warps == 1 || R <= 2) && !use_tc && split_warp_fits(pr->max_dim, pr->max_features, R);
   const SplitWs wl = split_ws(K, R, pr->max_dim, pr->max_features);
   if (!workspace || ws_bytes < wl.total) {
     set_error("art_split_level: workspace %zu bytes < required %zu", ws_bytes, wl.total);
@@ -2774,6 +1891,7 @@ extern "C" int art_split_level(const ArtSplitProblem* pr, const ArtSplitParams* 
     a.TC = 2;
     a.H = 1;
     a.gang_on = 0;
+    a.warp = 1;
   }
   if (cudaMemsetAsync(a.counts, 0, 4 * (kErrSlot + 1), s) != cudaSuccess) return check_launch("memset");
   if (a.gang_on &&
@@ -2788,27 +1906,7 @@ extern "C" int art_split_level(const ArtSplitProblem* pr, const ArtSplitParams* 
   prof_end(s);
   count_launch(); count_launch(); count_launch();
   if (use_warp) {
-    const size_t wsm = warp_layout(a.dmax, a.pmax).total;
-    auto launch_warp = [&](auto kern) -> int {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm) != cudaSuccess) {
-        cudaGetLastError();
-        set_error("art_split_level: cannot reserve %zu bytes of shared memory", wsm);
-        return ART_E_UNSUPPORTED;
-      }
-      const int occ = resident_ctas((const void*)kern, kWThreads, wsm);
-      const int64_t resident = (int64_t)device_sm_count() * std::max(occ, 1);
-      const int64_t grid = std::min<int64_t>(resident, (K * R + kWWarps - 1) / kWWarps);
-      prof_begin("split_level", s);
-      kern<<<(unsigned)std::max<int64_t>(grid, 1), kWThreads, wsm, s>>>(a);
-      prof_end(s);
-      count_launch();
-      return check_launch("split_level");
-    };
-    const int nbk = (a.pmax + 1 + 7) / 8;  // 8-column blocks of the widest psi
-    int rcw;
-    if (nbk == 1) rcw = launch_warp(split_warp_kernel<1>);
-    else if (nbk == 2) rcw = launch_warp(split_warp_kernel<2>);
-    else rcw = launch_warp(split_warp_kernel<3>);
+    const int rcw = launch_split_warp(a, s);
     if (rcw) return rcw;
     prof_begin("split_select", s);
     split_select<<<(unsigned)((K + 127) / 128), 128, 0, s>>>(a, *out);
