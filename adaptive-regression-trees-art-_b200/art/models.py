@@ -276,7 +276,7 @@ def solve_weighted_ridge_batched(
     ``tensor_min_features`` is the smallest feature count the mixed form
     solves on the tensor cores (smaller systems take the FP64 kernels); None
     takes the autotuned choice for this device and batch, else the library
-    default (48).
+    default (none).
     ``host_slices``: when ``x`` is in host memory (numpy, or a CPU tensor;
     pinned for the copies to run asynchronously) and the systems' rows are
     stored back to back, the batch is cut into this many slices of

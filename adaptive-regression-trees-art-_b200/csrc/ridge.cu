@@ -16,9 +16,9 @@
 //   ridge_dmma_kernel<6>, <3>              : FP64, (p+1) <= 48, warps alone on
 //       FP64 MMA Grams (ridge_dmma.cu); ridge_split_finish for the systems
 //       it split over several warps;
-//   ridge_fp64_kernel<8>                   : FP64, wider systems, persistent
-//       queue, 8x8 register tiles;
-//   ridge_fp64_kernel<8> on the resolve list (mixed systems that did not
+//   ridge_wide_kernel                      : FP64, wider systems, a CTA each
+//       (ridge_wide.cu);
+//   ridge_wide_kernel on the resolve list (mixed systems that did not
 //       converge); ridge_qr_kernel on the auto-solver fallback list.
 #include <stdarg.h>
 #include <stdio.h>
@@ -204,218 +204,7 @@ __global__ void __launch_bounds__(1024) ridge_plan_small(RidgeArgs a, RidgeLists
   }
 }
 
-// ============================================================ FP64 kernel
-// Shared-memory layout, identical on host and device.
-struct Fp64Layout {
-  int ldp;        // max padded augmented width
-  int chunk;
-  size_t off_x[2], off_y[2], off_w[2], off_bar, off_phi, off_q, off_gram, off_fa, off_fb,
-      off_vec, total;
-};
-
 __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
-
-// Position of feature blk*TS + j in a row of the sqrt(q)*phi tile of the
-// 8x8 register-tile form, and its row stride: within a block the entries
-// rotate by the block index, which spreads a warp's loads over the banks.
-__host__ __device__ inline int phi_pos(int ts, int blk, int j) { return blk * ts + ((j + blk) & (ts - 1)); }
-__host__ __device__ inline int phi_stride(int ts, int nb) { return nb * ts; }
-
-__host__ __device__ inline Fp64Layout fp64_layout(int pmax, int dmax, int ts, int chunk) {
-  Fp64Layout L;
-  const int pa = pmax + 1;
-  L.ldp = ((pa + ts - 1) / ts) * ts;  // features incl. padding
-  L.chunk = chunk;
-  size_t o = 0;
-  for (int s = 0; s < 2; ++s) {
-    L.off_x[s] = o; o = align16(o + (size_t)chunk * dmax * 8 + 16);
-    L.off_y[s] = o; o = align16(o + (size_t)chunk * 8 + 16);
-    L.off_w[s] = o; o = align16(o + (size_t)chunk * 8 + 16);
-  }
-  L.off_bar = o; o = align16(o + 2 * 8);
-  L.off_phi = o;
-  o = align16(o + (size_t)chunk * phi_stride(ts, L.ldp / ts) * 8);
-  L.off_q = o; o = align16(o + (size_t)chunk * 8);
-  L.off_gram = o; o = align16(o + (size_t)pa * (pa + 1) / 2 * 8);
-  L.off_fa = o; o = align16(o + (size_t)L.ldp * 2);
-  L.off_fb = o; o = align16(o + (size_t)L.ldp * 2);
-  L.off_vec = o; o = align16(o + (size_t)3 * (pa + 1) * 8);
-  L.total = o;
-  return L;
-}
-
-// Issue the bulk copies of chunk c (x rows, y, w) into stage st.
-__device__ __forceinline__ void issue_chunk(const RidgeArgs& a, const RidgeItem& it, int chunk,
-                                            int64_t c, unsigned char* smem, const Fp64Layout& lay,
-                                            int st, uint64_t* bar) {
-  const int64_t rr = c * chunk;
-  const int rows = (int)min((int64_t)chunk, it.n - rr);
-  Granules gx = granules(a.x + it.xoff + rr * it.d, (uint64_t)rows * it.d * 8);
-  Granules gy = granules(a.y + it.r0 + rr, (uint64_t)rows * 8);
-  Granules gw = a.w ? granules(a.w + it.r0 + rr, (uint64_t)rows * 8) : Granules{nullptr, 0, 0};
-  mbar_arrive_expect_tx(bar, gx.bytes + gy.bytes + gw.bytes);
-  bulk_g2s(smem + lay.off_x[st], gx.base, gx.bytes, bar);
-  bulk_g2s(smem + lay.off_y[st], gy.base, gy.bytes, bar);
-  if (a.w) bulk_g2s(smem + lay.off_w[st], gw.base, gw.bytes, bar);
-}
-
-template <int TS, int CHUNK>
-__global__ void __launch_bounds__(kRidgeThreads, 1) ridge_fp64_kernel(RidgeArgs a, RidgeLists L,
-                                                                   int cls, int pcap) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int s_item, s_fail;
-  __shared__ double s_scalar[4];
-  const Fp64Layout lay = fp64_layout(pcap, a.dmax, TS, CHUNK);
-  uint64_t* bars = (uint64_t*)(smem + lay.off_bar);
-  double* phi = (double*)(smem + lay.off_phi);
-  double* q = (double*)(smem + lay.off_q);
-  double* G = (double*)(smem + lay.off_gram);
-  int16_t* fa = (int16_t*)(smem + lay.off_fa);
-  int16_t* fb = (int16_t*)(smem + lay.off_fb);
-  double* vec = (double*)(smem + lay.off_vec);
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  uint32_t uses0 = 0, uses1 = 0;  // completed phases per stage (uniform)
-  const int count = L.count[cls];
-  for (;;) {
-    if (tid == 0) s_item = atomicAdd(&L.cursor[cls], 1);
-    __syncthreads();
-    const int item = s_item;
-    __syncthreads();
-    if (item >= count) break;
-    const int k = L.list[(int64_t)cls * a.K + item];
-    const RidgeItem it = load_item(a, k);
-    const int p = it.p, pa = p + 1, d = it.d;
-    const int nb = (pa + TS - 1) / TS;
-    const int ldpi = nb * TS;             // features incl. padding
-    const int lds = phi_stride(TS, nb);   // phi row stride
-    const int T = nb * (nb + 1) / 2;
-    const int S = max(1, kRidgeThreads / T);
-    for (int f = tid; f < ldpi; f += kRidgeThreads) {
-      int fa_, fb_;
-      if (f < p) feature_factors(d, it.kind, f, fa_, fb_);
-      else if (f == p) { fa_ = -2; fb_ = -1; }
-      else { fa_ = -3; fb_ = -1; }
-      fa[f] = (int16_t)fa_;
-      fb[f] = (int16_t)fb_;
-    }
-    const bool mine = tid < T * S;
-    const int tile = tid % T, slice = tid / T;
-    const int I = tile_row(tile), J = tile - I * (I + 1) / 2;
-    double acc[TS][TS];
-#pragma unroll
-    for (int i = 0; i < TS; ++i)
-#pragma unroll
-      for (int j = 0; j < TS; ++j) acc[i][j] = 0.0;
-    int bad = 0;
-    const int64_t nchunks = (it.n + CHUNK - 1) / CHUNK;
-    if (tid == 0) {
-      for (int64_t c = 0; c < min((int64_t)2, nchunks); ++c)
-        issue_chunk(a, it, CHUNK, c, smem, lay, (int)c, &bars[c]);
-    }
-    __syncthreads();  // fa/fb visible
-    bool timed_out = false;
-    int64_t timed_c = 0;
-    for (int64_t c = 0; c < nchunks; ++c) {
-      const int st = (int)(c & 1);
-      const uint32_t par = st ? (uses1 & 1) : (uses0 & 1);
-      const bool ok = mbar_wait(&bars[st], par);
-      if (!__syncthreads_and(ok)) { timed_out = true; timed_c = c; break; }
-      if (st) ++uses1; else ++uses0;
-      const int rows = (int)min((int64_t)CHUNK, it.n - c * CHUNK);
-      const double* xs =
-          (const double*)(smem + lay.off_x[st] +
-                          (((uintptr_t)(a.x + it.xoff + c * CHUNK * d)) & 15));
-      const double* ys =
-          (const double*)(smem + lay.off_y[st] + (((uintptr_t)(a.y + it.r0 + c * CHUNK)) & 15));
-      const double* ws =
-          a.w ? (const double*)(smem + lay.off_w[st] +
-                                (((uintptr_t)(a.w + it.r0 + c * CHUNK)) & 15))
-              : nullptr;
-      for (int e = tid; e < rows * d; e += kRidgeThreads) bad |= isfinite(xs[e]) ? 0 : 1;
-      for (int r = tid; r < rows; r += kRidgeThreads) {
-        bad |= isfinite(ys[r]) ? 0 : 1;
-        double wv = ws ? ws[r] : 1.0;
-        if (!(wv >= 0.0) || !isfinite(wv)) bad |= 2;
-        q[r] = sqrt(fmax(wv, a.weight_floor));
-      }
-      __syncthreads();
-      // phi[r][phi_pos(blk, j)] = sqrt(q_r) * feature(blk*TS + j): the
-      // rotation and shift spread the tiles' loads over distinct banks.
-      const int warp = tid >> 5, lane = tid & 31;
-      for (int r = warp; r < rows; r += kRidgeThreads / 32) {
-        const double* xr = xs + (int64_t)r * d;
-        const double sq = q[r];
-        for (int f = lane; f < ldpi; f += 32) {
-          const int ia = fa[f], ib = fb[f];
-          double v;
-          if (ia == -3) v = 0.0;
-          else if (ia == -2) v = sq * ys[r];
-          else v = sq * ((ia < 0 ? 1.0 : xr[ia]) * (ib < 0 ? 1.0 : xr[ib]));
-          const int blk = f / TS, j = f - blk * TS;
-          phi[r * lds + phi_pos(TS, blk, j)] = v;
-        }
-      }
-      __syncthreads();
-      if (tid == 0 && c + 2 < nchunks) issue_chunk(a, it, CHUNK, c + 2, smem, lay, st, &bars[st]);
-      if (mine) {
-        for (int r = slice; r < rows; r += S) {
-          const double* pr = phi + r * lds;
-          double av[TS], bv[TS];
-#pragma unroll
-          for (int i = 0; i < TS; ++i) av[i] = pr[phi_pos(TS, I, i)];
-#pragma unroll
-          for (int j = 0; j < TS; ++j) bv[j] = pr[phi_pos(TS, J, j)];
-#pragma unroll
-          for (int i = 0; i < TS; ++i)
-#pragma unroll
-            for (int j = 0; j < TS; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
-        }
-      }
-      __syncthreads();
-    }
-    if (timed_out) {
-      if (tid == 0) {
-        atomicExch(L.err, 1);
-        a.status[k] = -5;
-        // bounded waits for this CTA's own copies still in flight
-        for (int64_t c2 = timed_c; c2 < min(timed_c + 2, nchunks); ++c2) {
-          const int s2 = (int)(c2 & 1);
-          mbar_wait(&bars[s2], s2 ? (uses1 & 1) : (uses0 & 1));
-          if (s2) ++uses1; else ++uses0;
-        }
-      }
-      return;  // barrier phases are no longer consistent: stop this CTA
-    }
-    {
-      const int bw = __syncthreads_or(bad & 2), bx = __syncthreads_or(bad & 1);
-      bad = (bw ? 2 : 0) | (bx ? 1 : 0);
-    }
-    // deterministic slice reduction into the packed augmented Gram
-    for (int s = 0; s < S; ++s) {
-      if (mine && slice == s) {
-#pragma unroll
-        for (int i = 0; i < TS; ++i)
-#pragma unroll
-          for (int j = 0; j < TS; ++j) {
-            const int r = I * TS + i, cc = J * TS + j;
-            if (r < pa && cc <= r) {
-              double* g = &G[pk(r, cc)];
-              *g = (s == 0) ? acc[i][j] : *g + acc[i][j];
-            }
-          }
-      }
-      __syncthreads();
-    }
-    finish_fp64<TS>(a, L, k, it, G, bad, vec, &s_fail, s_scalar,
-                (cls == CLS_RESOLVE) ? ART_INFO_FP64_RESOLVE : 0u);
-  }
-}
 
 // ============================================================== QR kernel
 // FP64 Householder QR of the augmented least-squares problem
@@ -765,30 +554,6 @@ static SplitLayout split_layout(int64_t K, int max_features, size_t at) {
   return w;
 }
 
-template <typename Kern>
-static int launch_persistent(Kern kern, size_t smem, int64_t max_items, cudaStream_t s,
-                             RidgeArgs a, RidgeLists L, int cls, int pcap, const char* name) {
-  if (smem > 227 * 1024) {
-    set_error("%s: shared memory %zu bytes exceeds the 227 KB limit", name, smem);
-    return ART_E_UNSUPPORTED;
-  }
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    set_error("%s: cannot reserve %zu bytes of shared memory", name, smem);
-    return ART_E_UNSUPPORTED;
-  }
-  const int occ = resident_ctas((const void*)kern, kRidgeThreads, smem);
-  int64_t grid = (int64_t)device_sm_count() * occ;
-  if (grid > max_items) grid = max_items;
-  if (grid < 1) grid = 1;
-  prof_begin(name, s);
-  kern<<<(unsigned)grid, kRidgeThreads, smem, s>>>(a, L, cls, pcap);
-  prof_end(s);
-  count_launch();
-  return check_launch(name);
-}
-
 }  // namespace art
 
 using namespace art;
@@ -934,13 +699,10 @@ static int ridge_entry(const ArtRidgeProblem* pr, const ArtRidgeResult* res, flo
   }
   const bool tensor = a.precision == ART_PRECISION_MIXED && a.pmax >= a.tensor_min_p;
   if (a.pmax + 1 > kSmallMaxAug || tensor) {
-    const size_t sm = fp64_layout(a.pmax, a.dmax, 8, 32).total;
-    rc = launch_persistent(ridge_fp64_kernel<8, 32>, sm, K, s, a, L, CLS_LARGE, a.pmax,
-                           "ridge_fp64<8>");
+    rc = launch_ridge_wide(a, L, CLS_LARGE, s);
     if (rc) return rc;
     if (tensor) {
-      rc = launch_persistent(ridge_fp64_kernel<8, 32>, sm, K, s, a, L, CLS_RESOLVE, a.pmax,
-                             "ridge_fp64<8> resolve");
+      rc = launch_ridge_wide(a, L, CLS_RESOLVE, s);
       if (rc) return rc;
     }
   }

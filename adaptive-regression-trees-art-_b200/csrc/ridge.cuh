@@ -13,7 +13,7 @@ constexpr int kBuckets = 64;
 // to the last two.
 enum RidgeClass {
   CLS_SMALL = 0,    // FP64, 24 < (p+1) <= 48: warps alone, FP64 MMA Grams (ridge_dmma.cu)
-  CLS_LARGE = 1,    // FP64, (p+1) > 48: 8x8 register tiles
+  CLS_LARGE = 1,    // FP64, (p+1) > 48: a CTA each, FP64 MMA Grams (ridge_wide.cu)
   CLS_TENSOR = 2,   // mixed form, p at or above its threshold: tcgen05 split-product Gram
   CLS_WARP = 3,     // FP64, (p+1) <= 24: as CLS_SMALL, narrower blocks and more warps
   CLS_QR = 4,       // auto solver fallback: Householder QR
@@ -24,10 +24,12 @@ constexpr int kPlanClasses = 4;
 constexpr int kWarpMaxAug = 24;
 constexpr int kSmallMaxAug = 48;
 constexpr int kTensorMinP = 33;  // smallest p the tensor-core kernel takes
-// The mixed form's default threshold: below it the FP64 MMA kernel is the
-// faster one as well as the more exact (2,048 weighted systems of 306 to 8,192
-// rows and 45 features: 0.54 ms against 3.6 ms on the tensor-core kernel).
-constexpr int kTensorDefaultP = kSmallMaxAug;
+// The mixed form's default threshold: none.  The FP64 MMA kernels are the more
+// exact ones and at least as fast (weighted systems of 306 to 8,192 rows, FP64
+// against the tensor-core kernel: 2,048 of 45 features 0.54 and 3.6 ms; 510 of
+// 153 features 1.6 and 2.1 ms, 4,096 of them 12.2 and 12.2 ms, where its FP64
+// refinement passes over the rows cost what its Gram saves).
+constexpr int kTensorDefaultP = ART_MAX_FEATURES + 1;
 // Split systems (see ridge_dmma.cu): units per system at most, batches above
 // kSplitMaxCount systems are not split (they fill every warp by number).
 constexpr int kMaxUnits = 256;
@@ -137,130 +139,6 @@ __device__ __forceinline__ void write_failed(const RidgeArgs& a, int k, int p, i
   }
 }
 
-// Finish a system whose augmented Gram [G h; h^T yWy] is in packed lower
-// storage G (FP64, (p+1) rows) in shared memory: trace-scaled ridge, FP64
-// Cholesky, solve, optional condition estimate, and the auto-solver policy
-// of solve_weighted_ridge (models.py:268-371).  All threads call it.
-// `vec` is shared scratch of >= 3*(p+1) doubles.  Returns true if the system
-// was queued for the QR fallback.
-template <int CT>
-__device__ inline bool finish_fp64(const RidgeArgs& a, const RidgeLists& L, int k,
-                                   const RidgeItem& it, double* G, int bad, double* vec,
-                                   int* s_fail, double* s_scalar, uint32_t info0) {
-  const int tid = threadIdx.x, p = it.p;
-  const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  // lambda = ridge * trace(G) / p   (scaled_ridge_from_gram, models.py:209-215)
-  if (tid == 0) {
-    double tr = 0.0;
-    for (int i = 0; i < p; ++i) tr += G[pk(i, i)];
-    double lam = it.ridge * tr / p;
-    s_scalar[0] = lam;
-    L.lambda[k] = lam;
-  }
-  __syncthreads();
-  const double lam = s_scalar[0];
-  if (bad) {
-    write_failed(a, k, p, (bad & 2) ? -1 : -2, lam, info0);
-    __syncthreads();
-    return false;
-  }
-  if (a.solver == ART_SOLVER_QR || a.solver == ART_SOLVER_SVD) {  // explicit QR: no normal equations solve
-    if (tid == 0) {
-      if (a.ridge_eff) a.ridge_eff[k] = lam;
-      if (a.cond) a.cond[k] = nan;
-      if (a.info) a.info[k] = info0 | (a.solver == ART_SOLVER_SVD ? 0u : ART_INFO_QR_FALLBACK);
-      a.status[k] = 0;
-      push_list(L, a.K, CLS_QR, k);
-    }
-    __syncthreads();
-    return true;
-  }
-  for (int i = tid; i < p; i += blockDim.x) G[pk(i, i)] += lam;
-  __syncthreads();
-  const bool want_cond = (a.cond != nullptr) || (a.solver == ART_SOLVER_AUTO);
-  if (want_cond && tid < 32) {
-    double an = warp_sym_norm1(G, p);
-    if (tid == 0) s_scalar[1] = an;
-  }
-  __syncthreads();
-  // wide systems: 32-column blocks; narrow ones keep the small-register form
-  int fail;
-  if constexpr (CT == 8) fail = chol_packed32<double>(G, p, s_fail);
-  else fail = chol_packed<double, CT>(G, p, s_fail);
-  if (fail) {
-    if (a.solver == ART_SOLVER_AUTO) {
-      if (tid == 0) {
-        if (a.ridge_eff) a.ridge_eff[k] = lam;
-        if (a.cond) a.cond[k] = __longlong_as_double(0x7ff0000000000000ll);  // inf
-        if (a.info) a.info[k] = info0 | ART_INFO_QR_FALLBACK | ART_INFO_CHOLESKY_FAILED;
-        a.status[k] = 0;
-        push_list(L, a.K, CLS_QR, k);
-      }
-      __syncthreads();
-      return true;
-    }
-    write_failed(a, k, p, fail, lam, info0);
-    __syncthreads();
-    return false;
-  }
-  double* z = vec;
-  double* v = vec + (p + 1);
-  double* sg = vec + 2 * (p + 1);
-  if (tid < 32) {
-    for (int i = tid; i < p; i += 32) z[i] = G[pk(p, i)];  // h
-    __syncwarp();
-    warp_forward<double, double>(G, z, p);
-    warp_backward<double, double>(G, z, p);
-    if (want_cond) {
-      double est = warp_inv_norm1_estimate<double>(G, p, v, sg);
-      if (tid == 0) {
-        double an = s_scalar[1];
-        double rcond = (est > 0.0 && isfinite(est) && an > 0.0) ? 1.0 / (an * est) : 0.0;
-        s_scalar[2] = rcond;
-      }
-    }
-  }
-  __syncthreads();
-  uint32_t info = info0;
-  double cond = nan;
-  if (want_cond) {
-    double rcond = s_scalar[2];
-    if (rcond > 0.0 && isfinite(rcond)) {
-      cond = sqrt(1.0 / fmin(rcond, 1.0));
-    } else {
-      rcond = 0.0;
-      cond = __longlong_as_double(0x7ff0000000000000ll);
-      info |= ART_INFO_COND_FAILED;
-    }
-    if (a.solver == ART_SOLVER_AUTO && rcond < a.rcond_threshold) {
-      if (tid == 0) {
-        if (a.ridge_eff) a.ridge_eff[k] = lam;
-        if (a.cond) a.cond[k] = cond;
-        if (a.info) a.info[k] = info | ART_INFO_QR_FALLBACK | ART_INFO_RCOND_BELOW;
-        a.status[k] = 0;
-        push_list(L, a.K, CLS_QR, k);
-      }
-      __syncthreads();
-      return true;
-    }
-  }
-  int nonfinite = 0;
-  for (int i = tid; i < p; i += blockDim.x) {
-    double b = z[i];
-    nonfinite |= !isfinite(b);
-    a.beta[(int64_t)k * a.beta_stride + i] = b;
-  }
-  nonfinite = __syncthreads_or(nonfinite);
-  if (tid == 0) {
-    a.status[k] = nonfinite ? -3 : 0;
-    if (a.ridge_eff) a.ridge_eff[k] = lam;
-    if (a.cond) a.cond[k] = cond;
-    if (a.info) a.info[k] = info;
-  }
-  __syncthreads();
-  return false;
-}
-
 // Row of the lower-triangular tile grid holding linear tile index t.
 __device__ __forceinline__ int tile_row(int t) {
   int I = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
@@ -279,6 +157,7 @@ __device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
 
 // Host-side launch helpers (ridge.cu / ridge_tc.cu / ridge_dmma.cu).
 int launch_ridge_tensor(const RidgeArgs& a, const RidgeLists& L, cudaStream_t stream);
+int launch_ridge_wide(const RidgeArgs& a, const RidgeLists& L, int cls, cudaStream_t stream);
 int launch_ridge_dmma(const RidgeArgs& a, const RidgeLists& L, int cls, cudaStream_t stream);
 int launch_ridge_split_finish(const RidgeArgs& a, const RidgeLists& L, cudaStream_t stream);
 int ridge_dmma_ctas(int cls);

@@ -858,13 +858,14 @@ def run_b200(args):
     from art.models import kind_feature_count
 
     p_all = np.array([kind_feature_count(int(a), int(b)) for a, b in zip(wl.dims, wl.kinds)])
-    thr = args.tensor_min_features or (tuned["tensor_min_features"] if tuned else 48)
+    thr = args.tensor_min_features or (tuned["tensor_min_features"] if tuned else 161)
     if "dmma<3>" in name:
         cls_idx = np.flatnonzero(p_all + 1 <= 24)
     elif "dmma<6>" in name:
         cls_idx = np.flatnonzero((p_all + 1 > 24) & (p_all + 1 <= 48) & ((p_all < thr) | (args.precision == "fp64")))
-    elif "fp64<8>" in name:
-        cls_idx = np.flatnonzero(p_all + 1 > 48) if args.precision == "fp64" else np.flatnonzero(info & N.INFO_FP64_RESOLVE)
+    elif "ridge_wide" in name:
+        cls_idx = (np.flatnonzero(info & N.INFO_FP64_RESOLVE) if "resolve" in name else
+                   np.flatnonzero((p_all + 1 > 48) & ((p_all < thr) | (args.precision == "fp64"))))
     else:
         cls_idx = np.flatnonzero(p_all >= thr)
     flops, nbytes = algorithmic(wl, cls_idx)

@@ -138,7 +138,7 @@ typedef struct ArtRidgeProblem {
   uint32_t options;       /* ART_RIDGE_OPT_* bits                           */
   int32_t tensor_min_features; /* mixed form: systems with p >= this go to the
                                   tensor-core kernel, smaller ones to the FP64
-                                  kernels (0: 48; > 160: none)               */
+                                  kernels (0 or > 160: none)                 */
 } ArtRidgeProblem;
 
 /* Mixed form: factor the tensor-core Gram in FP64 instead of FP32 (fewer

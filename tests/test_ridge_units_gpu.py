@@ -104,3 +104,62 @@ def test_bad_input_in_a_split_system(bad):
     st = out.status.cpu().numpy()
     assert st[0] == (-1 if "weight" in bad else -2) and st[1] == 0
     assert np.all(np.isnan(out.beta.cpu().numpy()[0])) and np.all(np.isfinite(out.beta.cpu().numpy()[1]))
+
+
+# the wide kernel: group rows of one to five, several warps a group, the widest
+# model (its right-hand side apart), rows of 16- and 8-byte copies, long and
+# short chunks (d > 64 takes chunks of 16 rows)
+@pytest.mark.parametrize("kind,d", [(AFFINE, 47), (POLY2, 9), (AFFINE, 63), (POLY1_NOBIAS, 64), (AFFINE, 96), (POLY1_NOBIAS, 97),
+                                    (POLY2, 14), (POLY1_NOBIAS, 127), (POLY1_NOBIAS, 128), (POLY2, 16), (AFFINE, 158),
+                                    (POLY1_NOBIAS, 160)])
+@pytest.mark.parametrize("weighted", [True, False])
+def test_wide_systems(kind, d, weighted):
+    from art.models import kind_feature_count, solve_weighted_ridge_batched
+
+    rng = np.random.default_rng(7 * d + kind)
+    p = kind_feature_count(d, kind)
+    ns = [0, 3, p + 5, 2 * p + 1, 1024, 1091]
+    ro = np.concatenate([[0], np.cumsum(ns)])
+    X = rng.uniform(-1.0, 1.0, (ro[-1], d))
+    y = rng.normal(size=ro[-1])
+    w = rng.uniform(0.0, 1.0, ro[-1]) if weighted else None
+    K = len(ns)
+    out = solve_weighted_ridge_batched(X.reshape(-1), y, w, ro, [d] * K, [kind] * K, [1e-4] * K, weight_floor=0.0,
+                                       max_features=p, max_dim=d, condition=True)
+    beta, st = out.beta.cpu().numpy(), out.status.cpu().numpy()
+    assert st[0] == 1 and np.all(st[1:] == 0)
+    for k in range(1, K):
+        rows = slice(ro[k], ro[k + 1])
+        phi = _phi(X[rows], kind)
+        q = np.ones(ns[k]) if w is None else w[rows]
+        G = phi.T @ (phi * q[:, None])
+        A = G + 1e-4 * np.trace(G) / p * np.eye(p)
+        ref = np.linalg.solve(A, phi.T @ (q * y[rows]))
+        cond = np.linalg.cond(A)
+        assert np.linalg.norm(beta[k, :p] - ref) <= max(1e-12, 1e-14 * cond) * np.linalg.norm(ref), (k, ns[k])
+        # the estimate is of the 1-norm condition number's square root, from below, rarely by more than 3
+        est = float(out.cond_estimate[k])
+        c1 = np.sqrt(np.linalg.cond(A, 1))
+        assert c1 / 3 <= est <= c1 * (1 + 1e-6)
+
+
+@pytest.mark.parametrize("bad", ["x", "y", "weight"])
+def test_bad_input_in_a_wide_system(bad):
+    from art.models import solve_weighted_ridge_batched
+
+    rng = np.random.default_rng(4)
+    d, ns = 16, [700, 500]
+    ro = np.concatenate([[0], np.cumsum(ns)])
+    X, y, w = rng.uniform(-1, 1, (ro[-1], d)), rng.normal(size=ro[-1]), rng.uniform(0, 1, ro[-1])
+    if bad == "x":
+        X[690, 15] = np.inf
+        w[690] = 0.0
+    elif bad == "y":
+        y[3] = np.nan
+    else:
+        w[699] = -1.0
+    for precision in ("fp64", "mixed"):
+        out = solve_weighted_ridge_batched(X.reshape(-1), y, w, ro, [d] * 2, [POLY2] * 2, [1e-6] * 2, precision=precision,
+                                           max_features=153, max_dim=d)
+        st = out.status.cpu().numpy()
+        assert st[0] == (-1 if bad == "weight" else -2) and st[1] == 0
