@@ -69,11 +69,42 @@ __device__ __forceinline__ void split_dmma(double (&c)[2], double a, double b) {
       : "d"(a), "d"(b));
 }
 
+// e^x for |x| <= 51 (Cody & Waite, "Software Manual for the Elementary
+// Functions", 1980): x = k ln 2 + r with k rounded by the shift 1.5 * 2^52 and
+// ln 2 in two parts (42 binary places, and the rest), the Taylor series of e^r to r^13 (|r| <= ln 2 / 2: the rest
+// is below 5e-18), and k added to the exponent.  No branch, so that several
+// gates of a row run side by side (256 nodes of 16 restarts: 73.8 ms to 71.0).
+// Within 1.04 ulp; the gate below errs by at most 2.32 ulp and 0.524 rms over
+// [-50, 50], with exp() and a division by 2.32 and 0.530.
+__device__ __forceinline__ double exp51(double x) {
+  const double shift = 6755399441055744.0;
+  const double t = fma(x, 1.4426950408889634, shift);
+  const double k = t - shift;
+  double r = fma(k, -0.6931471805598903, x);
+  r = fma(k, -5.497923018708371e-14, r);
+  const double r2 = r * r;
+  // even and odd halves of the series, each by Horner's rule in r^2
+  double e = 1.0 / 479001600.0, o = 1.0 / 6227020800.0;
+  e = fma(e, r2, 1.0 / 3628800.0);
+  o = fma(o, r2, 1.0 / 39916800.0);
+  e = fma(e, r2, 1.0 / 40320.0);
+  o = fma(o, r2, 1.0 / 362880.0);
+  e = fma(e, r2, 1.0 / 720.0);
+  o = fma(o, r2, 1.0 / 5040.0);
+  e = fma(e, r2, 1.0 / 24.0);
+  o = fma(o, r2, 1.0 / 120.0);
+  e = fma(e, r2, 0.5);
+  o = fma(o, r2, 1.0 / 6.0);
+  // e^r = 1 + (r + r2 (e + r o))
+  const double q = fma(r2, fma(r, o, e), r) + 1.0;
+  return __hiloint2double(__double2hiint(q) + (__double2loint(t) << 20), __double2loint(q));
+}
+
 __device__ __forceinline__ double sigm(double s) {
   s = fmin(fmax(s, -50.0), 50.0);  // objectives.py:49-51
   // 1 / v, v in [1, 1 + e^50]: the hardware's approximation and three
   // Newton-Raphson steps, without a division's range checks
-  const double v = 1.0 + exp(-s);
+  const double v = 1.0 + exp51(-s);
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
   r = fma(r, fma(-v, r, 1.0), r);

@@ -605,15 +605,17 @@ struct SplitWarp {
       const int xr = row(X);
       double u, v, fl, fr;
       fits<false>(xr, u, v, fl, fr);
-      if (lane < rows) {
-        const double yv = sw[xr + d4 + 1];
-        const double pi = gate((u - z) * invT);
-        const double eL = yv - fl, eR = yv - fr;
-        const double eL2 = eL * eL, eR2 = eR * eR;
-        const double c = (eR2 - eL2) * pi * (1.0 - pi) * inv_n;
-        sl += (1.0 - pi) * eL2 + pi * eR2;
-        sa += c;
-        snr += pi >= 0.5 ? 1.0 : 0.0;
+      // lanes past the tile's rows run along and add nothing
+      const double yv = sw[xr + d4 + 1];
+      const double pi = gate((u - z) * invT);
+      const double eL = yv - fl, eR = yv - fr;
+      const double eL2 = eL * eL, eR2 = eR * eR;
+      const double c = (eR2 - eL2) * pi * (1.0 - pi) * inv_n;
+      const bool live = lane < rows;
+      sl += live ? (1.0 - pi) * eL2 + pi * eR2 : 0.0;
+      sa += live ? c : 0.0;
+      snr += live && pi >= 0.5 ? 1.0 : 0.0;
+      if (live) {
         const double2* x2 = (const double2*)(sw + xr);
 #pragma unroll
         for (int i = 0; i < DP; i += 4)
@@ -706,8 +708,8 @@ struct SplitWarp {
     return sqrt(wsum(s));
   }
 
-  // Frozen-model losses of candidates alpha[0 .. nc) at the current temperature.
-  __device__ __forceinline__ void search_pass(const double (&alpha)[kCand], int nc, double (&f)[kCand]) {
+  // Frozen-model losses of the candidates at the current temperature.
+  __device__ __forceinline__ void search_pass(const double (&alpha)[kCand], double (&f)[kCand]) {
     double inw[kCand], anw[kCand], zc[kCand], s[kCand];
 #pragma unroll
     for (int c = 0; c < kCand; ++c) {
@@ -720,16 +722,14 @@ struct SplitWarp {
       const int xr = row(X);
       double u, v, fl, fr;
       fits<true>(xr, u, v, fl, fr);
-      if (lane < rows) {
-        const double yv = sw[xr + d4 + 1];
-        const double eL = yv - fl, eR = yv - fr;
-        const double eL2 = eL * eL, eR2 = eR * eR;
+      const double yv = sw[xr + d4 + 1];
+      const double eL = yv - fl, eR = yv - fr;
+      const double eL2 = eL * eL, eR2 = eR * eR;
+      const bool live = lane < rows;
 #pragma unroll
-        for (int c = 0; c < kCand; ++c)
-          if (c < nc) {
-            const double pi = gate(fma(u, inw[c], fma(v, anw[c], -zc[c])) * invT);
-            s[c] += (1.0 - pi) * eL2 + pi * eR2;
-          }
+      for (int c = 0; c < kCand; ++c) {
+        const double pi = gate(fma(u, inw[c], fma(v, anw[c], -zc[c])) * invT);
+        s[c] += live ? (1.0 - pi) * eL2 + pi * eR2 : 0.0;
       }
     });
 #pragma unroll
@@ -882,7 +882,7 @@ __device__ __forceinline__ void SplitWarp<NB, SIDED>::run(int item) {
       al[0] = a_;
 #pragma unroll
       for (int c = 1; c < kCand; ++c) al[c] = al[c - 1] * P.rho;
-      search_pass(al, nc, f);
+      search_pass(al, f);
       int hit = -1;
 #pragma unroll
       for (int c = kCand - 1; c >= 0; --c) {
