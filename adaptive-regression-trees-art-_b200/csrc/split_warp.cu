@@ -594,12 +594,20 @@ struct SplitWarp {
   // Soft residual pass at theta: loss, gradient, n_right (pi >= 0.5), the
   // projected gradient, its norm and the directional derivative.
   __device__ __forceinline__ void resid_pass() {
-    constexpr int DP = NB <= 3 ? 8 * NB : 48;
+    // Gradient sum of c_r x_r: a lane's own row into one accumulator an input;
+    // with the wide form's inputs that is 48 of them and a final sum of 48 x 32,
+    // so there lane = input, and with 16 inputs or fewer lane groups take their
+    // own rows (149 nodes to 120,000 rows, d = 32 or quadratic of d = 8: 29.9 ms
+    // to 27.8; in the narrow form the own row is the faster: 71.0 ms to 74.0 for
+    // 256 nodes of 16 restarts).
+    constexpr int DP = NB <= 3 ? 8 * NB : 0;
+    const int group = d <= 8 ? 8 : (d <= 16 ? 16 : 32), col = lane & (group - 1);
+    const int row0 = lane & ~(group - 1);
     const double z = V(L.scal + SC_Z);
     const double inv_n = 1.0 / (double)n;
-    double g[DP];
+    double g[DP > 0 ? DP : 2];
 #pragma unroll
-    for (int i = 0; i < DP; ++i) g[i] = 0.0;
+    for (int i = 0; i < (DP > 0 ? DP : 2); ++i) g[i] = 0.0;
     double sl = 0.0, sa = 0.0, snr = 0.0;
     tiles(G.g, G.P, [&](int X, int rows) {
       const int xr = row(X);
@@ -615,7 +623,20 @@ struct SplitWarp {
       sl += live ? (1.0 - pi) * eL2 + pi * eR2 : 0.0;
       sa += live ? c : 0.0;
       snr += live && pi >= 0.5 ? 1.0 : 0.0;
-      if (live) {
+      if constexpr (DP == 0) {
+        // columns past the inputs are read from what follows and dropped
+        B(L.Q + lane) = live ? c : 0.0;
+        __syncwarp();
+        const int end = min(row0 + group, rows);
+        int at = X + row0 * rs + col;
+#pragma unroll 4
+        for (int r = row0; r < end; ++r) {
+          g[0] = fma(B(L.Q + r), sw[at], g[0]);
+          at += rs;
+        }
+        if (d > 32)
+          for (int r = 0; r < rows; ++r) g[1] = fma(B(L.Q + r), sw[X + r * rs + lane + 32], g[1]);
+      } else if (live) {
         const double2* x2 = (const double2*)(sw + xr);
 #pragma unroll
         for (int i = 0; i < DP; i += 4)
@@ -628,27 +649,27 @@ struct SplitWarp {
           }
       }
     });
-    // lanes' gradients added through shared memory, lane i taking input i
     const double ts = warp_sum(sl), ta = warp_sum(sa), tn = warp_sum(snr);
+    double t[2] = {g[0], g[1]};
+    if constexpr (DP == 0) {
+      for (int o = group; o < 32; o <<= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
+    } else {  // lanes' sums added through shared memory, lane i taking input i
 #pragma unroll
-    for (int i = 0; i < DP; ++i)
-      if (i < d) B(i * 33 + lane) = g[i];
-    __syncwarp();
-    double t[2] = {0.0, 0.0};
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const int i = lane + 32 * m;
-      if (i < d) {
+      for (int i = 0; i < DP; ++i)
+        if (i < d) B(i * 33 + lane) = g[i];
+      __syncwarp();
+      t[0] = t[1] = 0.0;
+      if (lane < d) {
         double s0 = 0.0, s1 = 0.0;
 #pragma unroll 8
         for (int q = 0; q < 32; q += 2) {
-          s0 += B(i * 33 + q);
-          s1 += B(i * 33 + q + 1);
+          s0 += B(lane * 33 + q);
+          s1 += B(lane * 33 + q + 1);
         }
-        t[m] = s0 + s1;
+        t[0] = s0 + s1;
       }
+      __syncwarp();
     }
-    __syncwarp();
 #pragma unroll
     for (int m = 0; m < 2; ++m)
       if (lane + 32 * m < d) B(lane + 32 * m) = t[m];
