@@ -24,10 +24,12 @@
 //                 alpha0 * rho^k built by repeated multiplication).
 // A select kernel then keeps, per node, the best restart as split() does.
 #include <algorithm>
+#include <cooperative_groups.h>
 
 #include "bulk.cuh"
 #include "common.cuh"
 #include "linalg.cuh"
+#include "rows.cuh"
 #include "split.cuh"
 #include "tcgen05.cuh"
 
@@ -1569,135 +1571,223 @@ __global__ void split_select(SplitArgs a, ArtSplitResult out) {
 // Device initialisation of theta0 when none is supplied: w ~ N(0, I) from
 // Philox keyed by (seed, node, restart), normalised; z = median(X w) by
 // selection (numpy's median: mean of the two middle values for even n).
-__global__ void split_init_theta(SplitArgs a, double* theta0, int64_t stride) {
-  const int64_t kr = blockIdx.x;
-  if (kr >= a.K * a.R) return;
+//
+// The median is a radix select on the order-preserving 64-bit image of the
+// doubles (sign bit flipped for positives, all bits flipped for negatives):
+// six digit passes of up to 11 bits narrow a prefix to the exact key of the
+// m-th smallest u, counting the rows that share the prefix.  What bounds it is
+// reading the rows.  A start's rows are dealt to the CTAs of a cluster, which
+// keep their keys in shared memory (rows past that form theirs again in each
+// pass) and add each other's counts through distributed shared memory; ranks
+// that a small node has no rows for leave at once.  The result is an order
+// statistic, the same for every cluster size.
+// 203 nodes of 300 to 65,000 rows, one start each: 3.27 ms with one CTA a
+// start, which read its rows seven times, 0.36 ms now.
+constexpr int kInitThreads = 512;
+constexpr int kInitKeys = 8192;      // keys a CTA keeps
+constexpr int kInitRankRows = 1024;  // rows a rank is worth
+constexpr int kInitBins = 2048;      // 4 a thread
+// Starts up to which a cluster of 8 is given to each: with nodes to 65,000 rows
+// 203 starts take 0.36 ms (1.47 with single CTAs), 812 1.31 (1.68), 1,024 1.67
+// (1.70), 1,624 2.59 (1.98).  Beyond, single CTAs fill the device.
+constexpr int64_t kInitClusterStarts = 1024;
+int init_cluster(int64_t starts) { return starts <= kInitClusterStarts ? 8 : 1; }
+
+__global__ void __launch_bounds__(kInitThreads)
+    split_init_theta(SplitArgs a, double* theta0, int64_t stride, int csize) {
+  extern __shared__ __align__(16) unsigned long long init_keys[];
+  __shared__ __align__(16) unsigned int hist[2][kInitBins];
+  __shared__ double w[ART_MAX_DIM + 8];
+  __shared__ long long s_part[kInitThreads / 32], s_m, s_cnt;
+  __shared__ unsigned long long s_pre, s_min;
+  namespace cg = cooperative_groups;
+  const int64_t kr = blockIdx.x / csize;
+  const int rank = (int)(blockIdx.x - kr * csize), tid = threadIdx.x, lane = tid & 31;
   const int64_t k = kr / a.R;
   const int d = a.dims[k];
   const int64_t r0 = a.row_offsets[k], n = a.row_offsets[k + 1] - r0;
-  const int64_t xoff = a.x_offsets[k];
-  __shared__ double w[ART_MAX_DIM + 1];
-  if (threadIdx.x == 0) {
-    double nrm2 = 0.0;
-    // counter: (node k, restart) or, with per-node keys, (restart, node key):
-    // the latter does not depend on the node's position in the batch
-    const int64_t rr = kr - k * a.R;
-    const uint64_t nk = a.node_keys ? a.node_keys[k] : 0ull;
-    for (int i = 0; i < d; i += 2) {
-      Philox4 r = a.node_keys
-                      ? philox4x32_10((uint32_t)rr, (uint32_t)nk, (uint32_t)i, (uint32_t)(nk >> 32) ^ 0x5eed0000u,
-                                      (uint32_t)a.prm.seed, (uint32_t)(a.prm.seed >> 32))
-                      : philox4x32_10((uint32_t)kr, (uint32_t)(kr >> 32), (uint32_t)i, 0x5eedu,
-                                      (uint32_t)a.prm.seed, (uint32_t)(a.prm.seed >> 32));
-      double z0, z1;
+  const int ranks = (int)min((int64_t)csize, max((n + kInitRankRows - 1) / kInitRankRows, (int64_t)1));
+  if (rank >= ranks) return;
+  cg::cluster_group cl = cg::this_cluster();
+  auto barrier = [&] {  // the ranks that stayed
+    if (csize > 1) cl.sync();
+    else __syncthreads();
+  };
+  const double* x = a.x + a.x_offsets[k];
+  for (int i = 2 * tid; i < ART_MAX_DIM + 8; i += 2 * kInitThreads) {
+    double z0 = 0.0, z1 = 0.0;
+    if (i < d) {
+      // counter: (node k, restart) or, with per-node keys, (restart, node key):
+      // the latter does not depend on the node's position in the batch
+      const int64_t rr = kr - k * a.R;
+      const uint64_t nk = a.node_keys ? a.node_keys[k] : 0ull;
+      const Philox4 r = a.node_keys
+                            ? philox4x32_10((uint32_t)rr, (uint32_t)nk, (uint32_t)i,
+                                            (uint32_t)(nk >> 32) ^ 0x5eed0000u, (uint32_t)a.prm.seed,
+                                            (uint32_t)(a.prm.seed >> 32))
+                            : philox4x32_10((uint32_t)kr, (uint32_t)(kr >> 32), (uint32_t)i, 0x5eedu,
+                                            (uint32_t)a.prm.seed, (uint32_t)(a.prm.seed >> 32));
       normal_pair(r, z0, z1);
-      w[i] = z0;
-      if (i + 1 < d) w[i + 1] = z1;
     }
+    w[i] = z0;
+    w[i + 1] = i + 1 < d ? z1 : 0.0;  // zero-padded
+  }
+  for (int b = tid; b < kInitBins; b += kInitThreads) hist[0][b] = 0u;
+  __syncthreads();
+  if (tid == 0) {
+    double nrm2 = 0.0;
     for (int i = 0; i < d; ++i) nrm2 += w[i] * w[i];
     double nrm = sqrt(nrm2);
     if (nrm <= 1e-12) { w[0] = 1.0; for (int i = 1; i < d; ++i) w[i] = 0.0; nrm = 1.0; }
     for (int i = 0; i < d; ++i) w[i] /= nrm;
+    s_min = ~0ull;
+    s_cnt = 0;
   }
   __syncthreads();
-  // median of u = X w by a radix select on the order-preserving 64-bit image
-  // of the doubles (sign bit flipped for positives, all bits flipped for
-  // negatives): six digit passes of up to 11 bits narrow a prefix to the
-  // exact key of the m-th smallest u, each pass recomputing u and counting
-  // the rows that share the prefix into a shared histogram.
-  constexpr int kBins = 2048;
-  __shared__ unsigned int hist[kBins];
-  __shared__ unsigned long long s_pre;
-  __shared__ long long s_m;
-  auto ukey = [](double v) -> unsigned long long {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-  };
-  auto from_ukey = [](unsigned long long k) -> double {
-    return __longlong_as_double((long long)((k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k));
-  };
-  auto u_of = [&](int64_t i) {
-    double u = 0.0;
-    for (int cc = 0; cc < d; ++cc) u = fma(a.x[xoff + i * d + cc], w[cc], u);
-    return u;
-  };
-  auto kth = [&](long long m) -> unsigned long long {
-    unsigned long long prefix = 0ull, mask = 0ull;
-    // digits (shift, width): bits 53..63, 42..52, 31..41, 20..30, 9..19, 0..8
-    for (int pass = 0; pass < 6; ++pass) {
-      const int sh = pass < 5 ? 53 - 11 * pass : 0;
-      const int width = pass < 5 ? 11 : 9;
-      const unsigned long long dmask = (1ull << width) - 1ull;
-      for (int b = threadIdx.x; b < kBins; b += blockDim.x) hist[b] = 0u;
-      __syncthreads();
-      for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const unsigned long long k = ukey(u_of(i));
-        if ((k & mask) == prefix) atomicAdd(&hist[(k >> sh) & dmask], 1u);
-      }
-      __syncthreads();
-      if (threadIdx.x < 32) {
-        // warp 0: lane l sums bins [64 l, 64 l + 64); an exclusive scan over
-        // the lanes finds the lane holding rank m, which scans its own bins
-        const int l = threadIdx.x;
-        long long part = 0;
-        for (int b = 64 * l; b < 64 * l + 64; ++b) part += hist[b];
-        long long incl = part;
-        for (int o = 1; o < 32; o <<= 1) {
-          const long long t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (l >= o) incl += t;
-        }
-        const long long excl = incl - part;
-        const unsigned hit = __ballot_sync(0xffffffffu, m >= excl && m < incl);
-        const int owner = hit ? __ffs(hit) - 1 : 31;
-        if (l == owner) {
-          long long mm = m - excl;
-          int b = 64 * l;
-          for (; b < 64 * l + 63; ++b) {
-            if (mm < (long long)hist[b]) break;
-            mm -= hist[b];
-          }
-          s_pre = prefix | ((unsigned long long)b << sh);
-          s_m = mm;
-        }
-      }
-      __syncthreads();
-      prefix = s_pre;
-      m = s_m;
-      mask |= dmask << sh;
-      __syncthreads();
-    }
-    return prefix;
-  };
   if (n == 0) {
-    if (threadIdx.x == 0) { for (int i = 0; i < d; ++i) theta0[kr * stride + i] = w[i]; theta0[kr * stride + d] = 0.0; }
+    if (tid == 0) { for (int i = 0; i < d; ++i) theta0[kr * stride + i] = w[i]; theta0[kr * stride + d] = 0.0; }
     return;
   }
-  const unsigned long long k1 = kth((n - 1) / 2);
+  auto from_ukey = [](unsigned long long v) -> double {
+    return __longlong_as_double((long long)((v >> 63) ? (v & 0x7FFFFFFFFFFFFFFFull) : ~v));
+  };
+  const int vec = row_vec(x, d);
+  auto key_of = [&](int64_t i) -> unsigned long long {
+    const double* xr = x + i * d;
+    double u = 0.0;
+    for (int c = 0; c < d; c += 8) {
+      double v[8];
+      load8(xr, c, d, vec, v);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) u = fma(v[q], w[c + q], u);
+    }
+    const unsigned long long b = (unsigned long long)__double_as_longlong(u);
+    return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+  };
+  // f(key) of this rank's rows: rows (j ranks + rank) 512 + tid
+  const int64_t step = (int64_t)ranks * kInitThreads, first = (int64_t)rank * kInitThreads + tid;
+  auto each = [&](auto f) {
+    int64_t i = first;
+    for (int j = tid; j < kInitKeys && i < n; j += kInitThreads, i += step) f(init_keys[j]);
+    for (; i < n; i += step) f(key_of(i));
+  };
+  {
+    int64_t i = first;
+#pragma unroll 4
+    for (int j = tid; j < kInitKeys; j += kInitThreads) {
+      if (i < n) init_keys[j] = key_of(i);
+      i += step;
+    }
+  }
+  unsigned long long prefix = 0ull, mask = 0ull;
+  long long m = (n - 1) / 2;
+  // digits (shift, width): bits 53..63, 42..52, 31..41, 20..30, 9..19, 0..8
+#pragma unroll 1
+  for (int pass = 0; pass < 6; ++pass) {
+    const int sh = pass < 5 ? 53 - 11 * pass : 0;
+    const unsigned long long dmask = pass < 5 ? 2047ull : 511ull;
+    unsigned int* h = hist[pass & 1];
+    each([&](unsigned long long v) {
+      if ((v & mask) == prefix) atomicAdd(&h[(v >> sh) & dmask], 1u);
+    });
+    barrier();  // counts complete; the other buffer's last readers are done
+    for (int b = tid; b < kInitBins; b += kInitThreads) hist[(pass + 1) & 1][b] = 0u;
+    // thread: four bins, summed over the ranks; the thread whose bins hold rank
+    // m of the prefix's rows finds the digit
+    uint4 c = make_uint4(0u, 0u, 0u, 0u);
+    for (int r = 0; r < ranks; ++r) {
+      const uint4* p = (const uint4*)h + tid;
+      const uint4 t = ranks > 1 ? *cl.map_shared_rank(p, r) : *p;
+      c.x += t.x;
+      c.y += t.y;
+      c.z += t.z;
+      c.w += t.w;
+    }
+    const long long part = (long long)c.x + c.y + c.z + c.w;
+    long long incl = part;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) s_part[tid >> 5] = incl;
+    __syncthreads();
+    long long before = incl - part;
+    for (int q = 0; q < (tid >> 5); ++q) before += s_part[q];
+    if (m >= before && m < before + part) {
+      long long mm = m - before;
+      int b = 4 * tid;
+      if (mm >= c.x) {
+        mm -= c.x, ++b;
+        if (mm >= c.y) {
+          mm -= c.y, ++b;
+          if (mm >= c.z) mm -= c.z, ++b;
+        }
+      }
+      s_pre = prefix | ((unsigned long long)b << sh);
+      s_m = mm;
+    }
+    __syncthreads();
+    prefix = s_pre;
+    m = s_m;
+    mask |= dmask << sh;
+  }
+  const unsigned long long k1 = prefix;
   const double v1 = from_ukey(k1);
   double v2 = v1;
   if (n % 2 == 0) {
     // the next order statistic: v1 again if more than n/2 keys are <= k1,
     // else the smallest u above v1
-    __shared__ unsigned long long s_min;
-    __shared__ long long s_cnt;
-    if (threadIdx.x == 0) { s_min = ~0ull; s_cnt = 0; }
-    __syncthreads();
     long long cnt = 0;
     unsigned long long mn = ~0ull;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-      const unsigned long long k = ukey(u_of(i));
-      if (k <= k1) ++cnt;
-      else if (k < mn) mn = k;
-    }
+    each([&](unsigned long long v) {
+      if (v <= k1) ++cnt;
+      else if (v < mn) mn = v;
+    });
     atomicAdd((unsigned long long*)&s_cnt, (unsigned long long)cnt);
     atomicMin(&s_min, mn);
-    __syncthreads();
-    v2 = s_cnt > n / 2 ? v1 : from_ukey(s_min);
+    barrier();
+    if (tid == 0 && rank == 0) {
+      for (int r = 1; r < ranks; ++r) {
+        s_cnt += *cl.map_shared_rank(&s_cnt, r);
+        s_min = min(s_min, *cl.map_shared_rank(&s_min, r));
+      }
+      v2 = s_cnt > n / 2 ? v1 : from_ukey(s_min);
+    }
   }
-  if (threadIdx.x == 0) {
+  if (tid == 0 && rank == 0) {
     for (int i = 0; i < d; ++i) theta0[kr * stride + i] = w[i];
     theta0[kr * stride + d] = (n % 2 == 0) ? 0.5 * (v1 + v2) : v1;
   }
+  barrier();  // no rank leaves while its counts are read
+}
+
+int launch_init_theta(const SplitArgs& a, double* theta0, cudaStream_t s) {
+  const int64_t starts = a.K * a.R;
+  const int c = init_cluster(starts);
+  const size_t smem = sizeof(unsigned long long) * kInitKeys;
+  if (cudaFuncSetAttribute(split_init_theta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return check_launch("split_init_theta");
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)c;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(starts * c));
+  cfg.blockDim = dim3(kInitThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  prof_begin("split_init_theta", s);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, split_init_theta, a, theta0, (int64_t)(ART_MAX_DIM + 1), c);
+  prof_end(s);
+  count_launch();
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    set_error("split_init_theta: %s", cudaGetErrorString(e));
+    return ART_E_LAUNCH;
+  }
+  return 0;
 }
 
 struct SplitWs {
@@ -1871,10 +1961,7 @@ extern "C" int art_split_level(const ArtSplitProblem* pr, const ArtSplitParams* 
   } else {
     a.theta0 = (double*)(ws + wl.theta0);
     a.theta0_stride = ART_MAX_DIM + 1;
-    prof_begin("split_init_theta", s);
-    split_init_theta<<<(unsigned)(K * R), 256, 0, s>>>(a, (double*)(ws + wl.theta0), ART_MAX_DIM + 1);
-    prof_end(s);
-    count_launch();
+    if (const int rc = launch_init_theta(a, (double*)(ws + wl.theta0), s)) return rc;
   }
   // CTA form without the tensor-core Gram, one or two restarts per CTA: side
   // Grams as FP64 MMA tiles when the (side, block) items fit the warps'
