@@ -62,7 +62,7 @@ constexpr int kWWarps = kWThreads / 32;
 constexpr int kCand = 4;               // Armijo candidates per search pass
 constexpr int kNarrowAug = 24, kNarrowDim = 23;
 constexpr int kWideAug = 48, kWideDim = 46;
-constexpr int kWideTile = 912;         // doubles of a row tile, d > 23
+constexpr int kWideTile = 1344;        // doubles of a row tile, d > 23: 32 rows to d = 40, then 24
 constexpr int kClusterCtas = 8;
 // Gangs, as log2 of n + 1 (the plan's buckets, so that larger gangs come first
 // in the queue).  With at most two restarts a node: a CTA from 1,023 rows, a
@@ -1032,8 +1032,12 @@ __device__ __forceinline__ void SplitWarp<NB, SIDED>::run(int item) {
 // small one on, each warp pops its own, warp 0 of the CTA that met it starting
 // with that one.  (One call site per model width keeps the search inlined and
 // its state in registers.)
+// CTAs an SM: the narrow form's state fits 168 registers a thread (4 of 128
+// spill: 79.5 ms instead of 71.0 at 16 restarts); the wide form's does not, and
+// two CTAs leave room for whole 32-row tiles (149 nodes to 120,000 rows: 27.3 ms
+// with three, 26.0 with two, 24.9 with tiles of 32 rows instead of 24).
 template <bool WIDE>
-__global__ void __launch_bounds__(kWThreads, 3) split_warp_kernel(const __grid_constant__ WArgs W) {
+__global__ void __launch_bounds__(kWThreads, WIDE ? 2 : 3) split_warp_kernel(const __grid_constant__ WArgs W) {
   __shared__ int s_q;
   const SplitArgs& a = W.a;
   cg::cluster_group cl = cg::this_cluster();
