@@ -50,84 +50,6 @@ def to_device(array, dtype=None, device=None):
     return t.from_numpy(arr).to(device=device, non_blocking=False).contiguous()
 
 
-# Staging through pinned memory: a pageable copy moves 17 GB/s here, threads
-# fill pinned chunks at 190 GB/s and those move at 53 GB/s.  A call holds at
-# most _CHUNKS chunks, which torch's allocator of pinned memory keeps for the
-# next call of any thread; nothing is shared between calls.
-_CHUNK = 2 << 20
-_CHUNKS = 3
-
-
-def _pinned(nbytes):
-    t = torch()
-    return t.empty(nbytes, dtype=t.uint8, pin_memory=True)
-
-
-def upload_rows(array, dtype=None, device=None):
-    """to_device for large host arrays, by pinned chunks: complete on the current
-    stream, not on others; the host array is free when it returns."""
-
-    t = torch()
-    device = require_cuda() if device is None else device
-    if isinstance(array, t.Tensor):
-        return to_device(array, dtype, device)
-    arr = np.ascontiguousarray(array, dtype=None if dtype is None else _np_dtype(dtype))
-    if arr.nbytes < _CHUNK or not arr.flags.writeable or t.get_num_threads() == 1:
-        return to_device(arr, dtype, device)
-    src = t.from_numpy(arr)
-    out = t.empty(src.shape, dtype=src.dtype, device=device)
-    flat, to = src.view(-1).view(t.uint8), out.view(-1).view(t.uint8)
-    slots = []
-    for k, at in enumerate(range(0, arr.nbytes, _CHUNK)):
-        n = min(_CHUNK, arr.nbytes - at)
-        if k < _CHUNKS:
-            slots.append([_pinned(_CHUNK), None])
-        buf, done = slot = slots[k % _CHUNKS]
-        if done is not None:
-            done.synchronize()
-        buf[:n].copy_(flat[at:at + n])
-        to[at:at + n].copy_(buf[:n], non_blocking=True)
-        if at + _CHUNKS * _CHUNK < arr.nbytes:
-            slot[1] = t.cuda.Event()
-            slot[1].record()
-    return out
-
-
-def pack(arrays, device=None):
-    """Host arrays as views of one device buffer, each at a 256-byte boundary, by
-    one copy on the current stream."""
-
-    t = torch()
-    device = require_cuda() if device is None else device
-    places, total = [], 0
-    for a in arrays:
-        places.append(total)
-        total += -(-a.nbytes // 256) * 256
-    host = _pinned(total)
-    for a, at in zip(arrays, places):
-        host[at:at + a.nbytes].numpy().view(a.dtype).reshape(a.shape)[...] = a
-    dev = t.empty(total, dtype=t.uint8, device=device)
-    dev.copy_(host, non_blocking=True)
-    return [dev[at:at + a.nbytes].view(t.from_numpy(a[:0]).dtype).view(a.shape) for a, at in zip(arrays, places)]
-
-
-def download(*tensors):
-    """numpy arrays of device tensors, with one wait for all of them."""
-
-    t = torch()
-    total = sum(x.numel() * x.element_size() for x in tensors)
-    if not 0 < total <= _CHUNKS * _CHUNK:
-        return [x.cpu().numpy() for x in tensors]
-    host, at, views = _pinned(total), 0, []
-    for x in tensors:  # widest elements first: every view is aligned
-        n = x.numel() * x.element_size()
-        views.append(host[at:at + n].view(x.dtype).view(x.shape))
-        views[-1].copy_(x, non_blocking=True)
-        at += n
-    t.cuda.current_stream().synchronize()
-    return [t.empty(v.shape, dtype=v.dtype).copy_(v).numpy() for v in views]
-
-
 def _np_dtype(torch_dtype):
     t = torch()
     return {

@@ -179,7 +179,7 @@ class RegressionTree:
         """(leaf index, prediction) for every row of X, computed on the GPU."""
 
         from . import _native as N
-        from ._device import download, pack, ptr, require_cuda, stream_handle, torch, upload_rows
+        from ._device import ptr, require_cuda, stream_handle, to_device, torch
 
         child, theta, coef, kinds, d, supported = self.flatten()
         if not supported:
@@ -188,22 +188,16 @@ class RegressionTree:
             raise ValueError(f"X must have {d} columns, got {X.shape[1]}.")
         t = torch()
         dev = require_cuda()
-        # table rows of whole 32-byte sectors: the walk reads them four doubles at a time
-        rows = [np.zeros((len(a), -(-a.shape[1] // 4) * 4)) for a in (theta, coef)]
-        for wide, a in zip(rows, (theta, coef)):
-            wide[:, :a.shape[1]] = a
-        xs = upload_rows(np.ascontiguousarray(X), t.float64, dev)
-        tables = pack((child, rows[0], rows[1], kinds), dev)
+        xs = to_device(np.ascontiguousarray(X), t.float64, dev)
+        tensors = [to_device(a, dt, dev) for a, dt in ((child, t.int32), (theta, t.float64), (coef, t.float64),
+                                                       (kinds, t.int32))]
         leaf = t.empty(X.shape[0], dtype=t.int32, device=dev)
         pred = t.empty(X.shape[0], dtype=t.float64, device=dev)
         lib = N.load_library()
-        if stream is not None:  # the copies are ordered on the current stream
-            t.cuda.current_stream().synchronize()
-        N.check(lib.art_tree_predict(int(d), child.shape[0], ptr(tables[0]), ptr(tables[1]), rows[0].shape[1],
-                                     ptr(tables[2]), rows[1].shape[1], ptr(tables[3]), X.shape[0], ptr(xs),
+        N.check(lib.art_tree_predict(int(d), child.shape[0], ptr(tensors[0]), ptr(tensors[1]), theta.shape[1],
+                                     ptr(tensors[2]), coef.shape[1], ptr(tensors[3]), X.shape[0], ptr(xs),
                                      ptr(leaf), ptr(pred), stream_handle(stream)), "art_tree_predict")
-        pred, leaf = download(pred, leaf)
-        return leaf, pred
+        return leaf.cpu().numpy(), pred.cpu().numpy()
 
     def predict_one(self, x: np.ndarray) -> float:
         return self.leaf_for_point(x).predict_one(x)
