@@ -73,6 +73,13 @@ def _leaf_kind(model) -> int:
     return -1
 
 
+def _sector_rows(n: int, columns: int) -> np.ndarray:
+    """Zeros (n, columns) in rows of whole 32-byte sectors: the device walk reads
+    such tables four doubles at a time."""
+
+    return np.zeros((n, -(-columns // 4) * 4))[:, :columns]
+
+
 class RegressionTree:
     """Prediction-only regression tree."""
 
@@ -137,14 +144,14 @@ class RegressionTree:
             kind = _leaf_kind(self.root.model)
             d = (len(coef) - 1) if kind in (0, 1) else None
         child = np.full((len(nodes), 2), -1, dtype=np.int32)
-        theta = np.zeros((len(nodes), (d or 1) + 1))
+        theta = _sector_rows(len(nodes), (d or 1) + 1)
         kinds = np.zeros(len(nodes), dtype=np.int32)
         pmax = 1
         for n in nodes:
             if isinstance(n, LeafNode):
                 c = getattr(n.model, "coef_", None)
                 pmax = max(pmax, len(c) if c is not None else 1)
-        coef = np.zeros((len(nodes), pmax))
+        coef = _sector_rows(len(nodes), pmax)
         supported = True
         for i, n in enumerate(nodes):
             if isinstance(n, SplitNode):
@@ -189,6 +196,7 @@ class RegressionTree:
         t = torch()
         dev = require_cuda()
         xs = to_device(np.ascontiguousarray(X), t.float64, dev)
+        theta, coef = theta.base, coef.base  # whole rows
         tensors = [to_device(a, dt, dev) for a, dt in ((child, t.int32), (theta, t.float64), (coef, t.float64),
                                                        (kinds, t.int32))]
         leaf = t.empty(X.shape[0], dtype=t.int32, device=dev)
