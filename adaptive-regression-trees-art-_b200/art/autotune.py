@@ -15,7 +15,7 @@ caller's own batch, with CUDA events on the launching stream:
   Armijo step sizes evaluated per trial pass (``trial_steps``) and the
   resident CTAs per SM (``ctas_per_sm``: one with the deepest row ring, or
   two with half the shared memory and a 128-register cap), or the
-  warp-per-restart form (``restart_warps``) with its trial steps; each
+  warp form (``restart_warps``, trial steps unused there); each
   candidate runs the sample level and the fastest is kept.
 
 Results live in an in-process table keyed by the device (name, SM count,
@@ -246,8 +246,9 @@ def split_candidates(R: int, max_backtracks: int, d: int = 0, p: int = 0,
 
     Two CTAs per SM are tried for groups of at most 8 restarts: a group of 16
     keeps 16 restarts' state per thread, which the 128-register cap spills.
-    The warp-per-restart form is tried when the level fits it (d and p at
-    most 23, no tensor-core Gram)."""
+    The warp form is tried when the level fits it (d and p at most 23, no
+    tensor-core Gram); with at most two restarts every shape without that Gram
+    runs it, up to d = 46 and p = 47."""
 
     groups = sorted({g for g in (R, 16, 8, 4, 2, 1) if 1 <= g <= min(R, 16)}, reverse=True)
     out = []

@@ -37,7 +37,7 @@ import numpy as np
 from . import _native as N
 from .autotune import WARP_MAX_DIM, WARP_MAX_FEATURES
 
-WARP_MAX_ROWS = 1 << 16  # split nodes up to this size take the warp-per-restart form
+WARP_MAX_ROWS = 1 << 16  # split nodes up to this size share the narrow launch
 from ._device import ptr, require_cuda, stream_handle, torch
 from .models import AffineRidgeModel, segment_residuals, solve_weighted_ridge_batched
 from .splitters import SoftObliqueSplitter, split_level
@@ -362,16 +362,12 @@ class ServingEngine:
                 st.leaves.append(nd)
             else:
                 split_idx.append(k)
-        # (The CTA form runs two CTAs per SM here: many small single-restart
-        # nodes keep one CTA per SM waiting at its barriers; 1.34x on a level
-        # of 4,609 such d = 32 nodes.)
         # max_iters is a per-call parameter of the split search (one call per
         # distinct value); the minimum side count goes per node, so nodes of
-        # every dimension share a launch.  Nodes for the warp-per-restart form
-        # (d and p at most 23, at most WARP_MAX_ROWS rows: larger nodes take
-        # the CTA form, whose gangs span many SMs) and the others go to
-        # separate launches, since the form of a launch is one for all its
-        # nodes: so a node's split never depends on the nodes batched with it.
+        # every dimension share a launch.  Narrow nodes (d and p at most 23, at
+        # most WARP_MAX_ROWS rows) and the others go to separate launches: a
+        # launch's kernel follows its widest node, and the narrow one keeps more
+        # warps on an SM.  A node's split is the same in either.
         groups: dict[tuple[int, bool], list[int]] = {}
         for k in split_idx:
             job = work[k][0].job
