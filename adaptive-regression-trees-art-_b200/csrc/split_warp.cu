@@ -14,7 +14,8 @@
 //   Gram pass     : both sides' weighted Grams at the accepted theta and the
 //                   temperature that follows it.
 //
-// What bounds it: the FP64 pipe and, with few items, the latency of a pass.
+// What bounds it: the latency of dependent FP64 chains at 12 (narrow) or 8
+// (wide) warps an SM and, with few items, that of a pass.
 // The Grams run as mma.sync m8n8k4 f64 (16 cycles of a scheduler's FP64 pipe
 // each); scores, fitted values, gradient and gates are per-row lane work,
 // because as MMAs most of their columns would be padding (the three score
@@ -35,11 +36,10 @@
 // the number of restarts, the call's parameters, never the batch.
 //
 // Against one trial with its Gram per pass and gangs of one CTA (B200): one
-// node of 4,096 rows, d = 2, 24 iterations 3.0 -> 0.41 ms; 203 nodes of 300 to
-// 65,000 rows, one restart, 166 -> 11.5 ms; 256 nodes x 16 restarts, d = 16, 30
-// iterations 140 -> 73 ms.  149 nodes of 300 to 120,000 rows with 33 or 45
-// features, before in the CTA form, 270 -> 30 ms.  Sixteen warps an SM instead
-// of twelve (a 128-register cap) spilled: 87 ms for the 16-restart level.
+// node of 4,096 rows, d = 2, 24 iterations 3.0 -> 0.37 ms; 203 nodes of 300 to
+// 65,000 rows, one restart, 153 -> 11.4 ms with the starts; 256 nodes x 16
+// restarts, d = 16, 30 iterations 140 -> 70 ms.  149 nodes of 300 to 120,000 rows
+// with 33 or 45 features, before in the CTA form, 268 -> 24 ms.
 //
 // Models of more than 23 features keep one side's Gram blocks per warp: the
 // warps of a pair take the same tiles in the Gram passes, one side each, and
