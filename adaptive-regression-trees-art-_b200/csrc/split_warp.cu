@@ -1150,6 +1150,8 @@ __global__ void __launch_bounds__(kWThreads, WIDE ? 2 : 3) split_warp_kernel(con
   const int count = a.counts[0];
   const int cta_log = a.R <= 2 ? kCtaLogFew : kCtaLogMany;
   int phase = W.csize > 1 ? 0 : 1;  // 0: cluster, 1: CTA, 2: warp
+  // every CTA of the cluster has started before one writes to another's memory
+  if (phase == 0) cl.sync();
   for (;;) {
     int q = -1;
     Gang g{1, 0, false};
