@@ -9,6 +9,8 @@
 // |w . x - z|.
 #include <cooperative_groups.h>
 
+#include <utility>
+
 #include "common.cuh"
 #include "rows.cuh"
 
@@ -280,6 +282,9 @@ __global__ void __launch_bounds__(kLevelThreads)
                     int64_t bs, double* sse, double* ssy) {
   cg::cluster_group cluster = cg::this_cluster();
   const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
+  // CTA 0 has started before its shared memory is written: waited for once the
+  // coefficients are in place
+  auto started = cluster.barrier_arrive();
   const int64_t k = blockIdx.x / csize;
   const int64_t r0 = seg.row_offsets[k], n = seg.row_offsets[k + 1] - r0;
   const int64_t xoff = seg.x_offsets[k];
@@ -308,6 +313,7 @@ __global__ void __launch_bounds__(kLevelThreads)
   const int vec = row_vec(xk, d);
   const int ranks = (int)min((int64_t)kMaxRanks, (n + 1023) / 1024);
   const int64_t span = ranks ? (n + ranks - 1) / ranks : 0;
+  cluster.barrier_wait(std::move(started));
   for (int v = crank; v < ranks; v += csize) {
     const int64_t a = span * v, b = min(n, a + span);
     double s_e = 0.0, s_y = 0.0;

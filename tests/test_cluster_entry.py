@@ -20,7 +20,7 @@ def _functions(text):
     return [body for body in re.split(r"^\};?\s*$", text, flags=re.M) if "map_shared_rank" in body]
 
 
-@pytest.mark.parametrize("source", ["split.cu", "split_warp.cu"])
+@pytest.mark.parametrize("source", ["split.cu", "split_warp.cu", "tree.cu"])
 def test_a_cluster_barrier_precedes_the_first_remote_access(source):
     bodies = _functions((CSRC / source).read_text())
     assert bodies
