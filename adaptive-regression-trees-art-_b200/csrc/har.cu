@@ -161,10 +161,11 @@ __device__ __forceinline__ bool team_any(bool v) {
   return ((m >> (lane / TL * TL)) & (TL == 32 ? 0xffffffffu : (1u << (TL & 31)) - 1u)) != 0;
 }
 
-// Shared memory of a team, in doubles: A [cap][d], the directions [bufs][SB][us],
+// Shared memory of a team, in doubles: A [cap][us], the directions [bufs][SB][us],
 // the products [SB][as], the uniforms [bufs][SB], the state [d].  Odd strides
-// us and as put the lanes of part 2 (one step each) into different banks; the
-// team stride, 8 modulo 16, does the same for the teams of a warp.
+// us and as put the lanes of part 2 (one step each), and in the slacks those
+// with a row each, into different banks; the team stride, 8 modulo 16, does the
+// same for the teams of a warp.
 struct HarLayout {
   int us, as, bufs;
   int U, AU, UN, X, total;
@@ -174,7 +175,7 @@ __host__ __device__ inline HarLayout har_layout(int d, int cap, int SB, bool inj
   L.us = d | 1;
   L.as = cap | 1;
   L.bufs = injected || maps ? 2 : 1;  // the next block's draws in flight, or z beside u = M z
-  L.U = cap * d;
+  L.U = cap * L.us;
   L.AU = L.U + L.bufs * SB * L.us;
   L.UN = L.AU + SB * L.as;
   L.X = L.UN + L.bufs * SB;
@@ -221,12 +222,12 @@ __global__ void __launch_bounds__(kHarThreads) har_kernel(HarArgs a) {
     slo[m] = x[m] - lo_[m];
     if (own) Xs[i] = x[m];
   }
-  for (int e = lane; e < a.cap * d; e += TL) As[e] = e < k * d ? a.A[rb * d + e] : 0.0;
+  for (int e = lane; e < a.cap * d; e += TL) As[e / d * L.us + e % d] = e < k * d ? a.A[rb * d + e] : 0.0;
   __syncwarp();
   auto row_slack = [&](int m) {  // b - A x of this lane's m-th row
     const int r = lane + TL * m;
     if (r >= k) return 0.0;
-    return __dsub_rn(br[m], pair_tree<H>(As + r * d, Xs, d));
+    return __dsub_rn(br[m], pair_tree<H>(As + r * L.us, Xs, d));
   };
   bool bad = false;
 #pragma unroll
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(kHarThreads) har_kernel(HarArgs a) {
         UN[st] = a.unif[(int64_t)chain * total + at];
       }
     }
-    for (int r = part; r < k; r += NP) AUs[st * L.as + r] = pair_tree<H>(As + r * d, U + st * L.us, d);
+    for (int r = part; r < k; r += NP) AUs[st * L.as + r] = pair_tree<H>(As + r * L.us, U + st * L.us, d);
     __syncwarp();
     // ---- 3. lane = constraint: the steps in order
     double nu[CPL], niu[CPL], nau[RPL], nia[RPL], nun;
