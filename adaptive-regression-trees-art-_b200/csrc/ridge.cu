@@ -81,18 +81,18 @@ __device__ __forceinline__ int plan_item(const RidgeArgs& a, int64_t k, bool rep
 // warp's share of its class and the pool has room, as a split system (a run
 // of units per queue entry, about a quarter of a share each).  `slot` is the
 // list position it would take; a split item leaves its place to a zero-cost
-// marker (-1).
+// marker (-1), one that the pool has no room for is marked (-2 - k).
 __device__ void plan_place(const RidgeArgs& a, const RidgeLists& L, int64_t k, int c, int slot, int64_t n, int p) {
   const int sc = split_class(c);
   int32_t entry = (int32_t)k;
-  if (sc >= 0 && L.pool_cap > 0) {
+  if (sc >= 0) {
     const int pa = p + 1, E = pa * (pa + 1) / 2;
     const int64_t U = ridge_unit_rows(n);
     const int nseg = (int)((n + U - 1) / U);
     const unsigned long long share = __ldcg(&L.cost[sc]) / (unsigned)max(L.workers[sc], 1);
     if (nseg > 1 && split_cost(n, pa) > share) {
       const unsigned long long need = (unsigned long long)nseg * E;
-      const unsigned long long at = atomicAdd(L.pool_used, need);
+      const unsigned long long at = L.pool_cap > 0 ? atomicAdd(L.pool_used, need) : 0;
       if (at + need <= (unsigned long long)L.pool_cap) {
         const int r = atomicAdd(L.nrec, 1);
         if (r < L.rec_cap) {
@@ -111,6 +111,10 @@ __device__ void plan_place(const RidgeArgs& a, const RidgeLists& L, int64_t k, i
           L.recs[r] = rec;
           if (fits) entry = -1;
         }
+      }
+      if (entry >= 0 && c == CLS_SMALL) {  // no room: a CTA's
+        entry = -2 - entry;
+        atomicAdd(L.nshared, 1);
       }
     }
   }
@@ -645,6 +649,7 @@ static int ridge_entry(const ArtRidgeProblem* pr, const ArtRidgeResult* res, flo
   L.list = (int32_t*)(ws + wl.off_list);
   L.nrec = L.err + 1;
   L.nitems = L.err + 2;
+  L.nshared = L.err + 10;
   L.cost = (unsigned long long*)(L.err + 4);
   L.pool_used = L.cost + 2;
   const SplitLayout sl = split_layout(K, a.pmax, wl.total);

@@ -96,6 +96,7 @@ struct RidgeLists {
   unsigned long long* pool_used;  // doubles taken from the pool
   int32_t* nrec;    // records taken
   int32_t* nitems;  // [2] queue entries: (record, first unit, units)
+  int32_t* nshared; // CLS_SMALL systems marked for a whole CTA: list entry -2 - k
   SplitRec* recs;
   int4* items;      // [2][item_cap]
   double* pool;

@@ -164,10 +164,12 @@ __device__ void warp_finish(const RidgeArgs& a, const RidgeLists& L, int k, int 
 
 // One warp's work on units [u0, u0 + nu) of system k.  `part` (the system's
 // pool slots) receives each unit's Gram of a split system; without it the
-// units' sum is left in the warp's G.  QUAD: the quadratic kinds (two factors
-// a feature, fixed row stride).  Returns the input-check bits.
+// units' sum is left in the warp's G, `add`ed to what it holds.  QUAD: the
+// quadratic kinds (two factors a feature, fixed row stride).  Returns the
+// input-check bits.
 template <int MAXNB, int NB, bool QUAD>
-__device__ int gram_units(const RidgeArgs& a, const RidgeItem& it, unsigned char* base, int u0, int nu, double* part) {
+__device__ int gram_units(const RidgeArgs& a, const RidgeItem& it, unsigned char* base, int u0, int nu, double* part,
+                          bool add) {
   using T = DmTraits<MAXNB>;
   using Lay = DmLayout<MAXNB>;
   constexpr int NBLK = NB * (NB + 1) / 2;
@@ -296,7 +298,7 @@ __device__ int gram_units(const RidgeArgs& a, const RidgeItem& it, unsigned char
         for (int64_t e = ra + lane; e < unit_end; e += 32) bad |= isfinite(a.y[it.r0 + e]) ? 0 : 1;
       }
       double* dst = part ? part + (size_t)unit * E : G;
-      const bool first = part || unit == u0;
+      const bool first = part || (unit == u0 && !add);
 #pragma unroll
       for (int I = 0; I < NB; ++I)
 #pragma unroll
@@ -319,20 +321,61 @@ __device__ int gram_units(const RidgeArgs& a, const RidgeItem& it, unsigned char
   return __reduce_or_sync(0xffffffffu, bad);
 }
 
+// Several warps' Grams of consecutive units added in unit order, by all threads
+// of the CTA: warp 0's holds the units before, and its own.
+template <int MAXNB>
+__device__ void add_grams(unsigned char* smem, int E, int n) {
+  using Lay = DmLayout<MAXNB>;
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += kDmThreads) {
+    double* g = (double*)(smem + Lay::kG) + e;
+    double t = *g;
+    for (int w = 1; w < n; ++w) t += g[w * (Lay::kPerWarp / 8)];
+    *g = t;
+  }
+  __syncthreads();
+}
+
 // MAXNB = 3: p + 1 <= 24 at 16 warps per SM; 6: p + 1 <= 48 at 12 warps.
+//
+// A wide-class system that costs more than a warp's share, but has no room in
+// the pool (no workspace for one, or a batch too long to be split), is the
+// whole CTA's: its warps take every fourth unit.  Marked entries stand at the
+// head of the list, largest first, so a CTA takes entries one at a time until
+// it meets an unmarked one; warps that meet a marked one later walk it alone.
+// One system of 100,000 rows and 47 features: 13.25 ms by one warp, 3.5 ms here;
+// one of 200,000 among 17,000 of 60 rows: 26.3 ms and 7.1.
 template <int MAXNB>
 __global__ void __launch_bounds__(kDmThreads, MAXNB == 3 ? 4 : 3) ridge_dmma_kernel(RidgeArgs a, RidgeLists L, int cls) {
   extern __shared__ __align__(128) unsigned char smem[];
   using Lay = DmLayout<MAXNB>;
+  __shared__ int s_q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* base = smem + (size_t)warp * Lay::kPerWarp;
   const int sc = cls == CLS_WARP ? 0 : 1;
   const int count = L.count[cls], nsplit = min(L.nitems[sc], L.item_cap);
+  bool together = MAXNB > 3 && *L.nshared > 0;
   for (;;) {
     int q = 0;
-    if (lane == 0) q = atomicAdd(&L.cursor[cls], 1);
-    q = __shfl_sync(0xffffffffu, q, 0);
-    if (q >= nsplit + count) break;
+    bool shared = false;
+    if (MAXNB > 3 && together) {
+      __syncthreads();
+      if (threadIdx.x == 0) s_q = atomicAdd(&L.cursor[cls], 1);
+      __syncthreads();
+      q = s_q;
+      if (q >= nsplit + count) break;
+      const int k = q < count ? L.list[(int64_t)cls * a.K + q] : -1;
+      shared = k < -1;
+      if (q < count && k == -1) continue;
+      if (!shared) {
+        together = false;
+        if (warp != 0) continue;
+      }
+    } else {
+      if (lane == 0) q = atomicAdd(&L.cursor[cls], 1);
+      q = __shfl_sync(0xffffffffu, q, 0);
+      if (q >= nsplit + count) break;
+    }
     int k, u0 = 0, nu = 1 << 30, rec = -1;
     double* part = nullptr;
     if (q >= count) {  // a run of units of a split system: a quarter of a share each, so they come last
@@ -345,28 +388,47 @@ __global__ void __launch_bounds__(kDmThreads, MAXNB == 3 ? 4 : 3) ridge_dmma_ker
       part = L.pool + L.recs[rec].base;
     } else {
       k = L.list[(int64_t)cls * a.K + q];
-      if (k < 0) continue;  // split
+      if (k == -1) continue;  // split
+      if (k < 0) k = -2 - k;  // marked
     }
     const RidgeItem it = load_item(a, k);
-    const int U = (int)ridge_unit_rows(it.n);
-    nu = min(nu, (int)((it.n + U - 1) / U));
+    const int U = (int)ridge_unit_rows(it.n), units = (int)((it.n + U - 1) / U);
+    nu = min(nu, units);
     const int nb = (it.p + 1 + 7) / 8;
     // (a nonlinear kind has its x among the features of the first two blocks:
     // p <= 47 means d <= 8)
     const bool quad = it.kind == ART_FEATURES_POLY2 || it.kind == ART_FEATURES_POLY2_NOBIAS;
-    int bad;
-    if constexpr (MAXNB == 3) {
-      if (nb == 1) bad = quad ? gram_units<3, 1, true>(a, it, base, u0, nu, part) : gram_units<3, 1, false>(a, it, base, u0, nu, part);
-      else if (nb == 2) bad = quad ? gram_units<3, 2, true>(a, it, base, u0, nu, part) : gram_units<3, 2, false>(a, it, base, u0, nu, part);
-      else bad = quad ? gram_units<3, 3, true>(a, it, base, u0, nu, part) : gram_units<3, 3, false>(a, it, base, u0, nu, part);
-    } else {
-      if (nb <= 4) bad = quad ? gram_units<6, 4, true>(a, it, base, u0, nu, part) : gram_units<6, 4, false>(a, it, base, u0, nu, part);
-      else if (nb == 5) bad = quad ? gram_units<6, 5, true>(a, it, base, u0, nu, part) : gram_units<6, 5, false>(a, it, base, u0, nu, part);
-      else bad = quad ? gram_units<6, 6, true>(a, it, base, u0, nu, part) : gram_units<6, 6, false>(a, it, base, u0, nu, part);
+    const int rounds = shared ? (units + kDmWarps - 1) / kDmWarps : 1;
+    int bad = 0;
+#pragma unroll 1
+    for (int r = 0; r < rounds; ++r) {
+      bool add = false;
+      if (shared) {
+        u0 = kDmWarps * r + warp;
+        nu = 1;
+        add = warp == 0 && r > 0;
+      }
+      int b;
+      if constexpr (MAXNB == 3) {
+        if (nb == 1) b = quad ? gram_units<3, 1, true>(a, it, base, u0, nu, part, add) : gram_units<3, 1, false>(a, it, base, u0, nu, part, add);
+        else if (nb == 2) b = quad ? gram_units<3, 2, true>(a, it, base, u0, nu, part, add) : gram_units<3, 2, false>(a, it, base, u0, nu, part, add);
+        else b = quad ? gram_units<3, 3, true>(a, it, base, u0, nu, part, add) : gram_units<3, 3, false>(a, it, base, u0, nu, part, add);
+      } else {
+        if (nb <= 4) b = quad ? gram_units<6, 4, true>(a, it, base, u0, nu, part, add) : gram_units<6, 4, false>(a, it, base, u0, nu, part, add);
+        else if (nb == 5) b = quad ? gram_units<6, 5, true>(a, it, base, u0, nu, part, add) : gram_units<6, 5, false>(a, it, base, u0, nu, part, add);
+        else b = quad ? gram_units<6, 6, true>(a, it, base, u0, nu, part, add) : gram_units<6, 6, false>(a, it, base, u0, nu, part, add);
+      }
+      bad |= b;
+      if (shared) add_grams<MAXNB>(smem, (it.p + 1) * (it.p + 2) / 2, min(kDmWarps, units - kDmWarps * r));
     }
     if (rec >= 0) {
       if (bad && lane == 0) atomicOr(&L.recs[rec].bad, bad);
       continue;
+    }
+    if (shared) {
+      const int bw = __syncthreads_or(bad & 2), bx = __syncthreads_or(bad & 1);
+      if (warp != 0) continue;
+      bad = (bw ? 2 : 0) | (bx ? 1 : 0);
     }
     warp_finish<MAXNB <= 3 ? 1 : 2>(a, L, k, it.p, it.ridge, (double*)(base + Lay::kG), bad, (double*)base,
                                     DmTraits<MAXNB>::kPad + 1);
