@@ -241,10 +241,12 @@ __global__ void __launch_bounds__(kPredictThreads)
 // node's rows are cut into up to kMaxRanks ranges, fixed by its row count;
 // each range is one CTA's sum (threads in row order, then a fixed tree), and
 // the ranges are added in order.
+//
+// The features' products are formed and added in feature order, as
+// feature_factors gives it: the nested form x_i (b_i + sum b_ij x_j) has fewer
+// operations but other roundings, and overflows where the products do not.
 template <int DP>
 __device__ __forceinline__ double quad_predict(const double* xr, const double* q, int d, int vec) {
-  // nested form of the quadratic: x_i (b_i + sum_{j >= i} b_ij x_j), the
-  // coefficients zero-padded to DP inputs: [b_0 | DP linear | DP (DP + 1) / 2]
   double v[DP];
 #pragma unroll
   for (int i = 0; i < DP; i += 8) {
@@ -254,25 +256,35 @@ __device__ __forceinline__ double quad_predict(const double* xr, const double* q
     for (int u = 0; u < 8; ++u) v[i + u] = t[u];
   }
   double s = q[0];
-  int f = 1 + DP;
+  int f = 1;
 #pragma unroll
-  for (int i = 0; i < DP; ++i) {
-    double t = q[1 + i];
+  for (int i = 0; i < DP; ++i) s = fma(v[i], q[f++], s);
 #pragma unroll
-    for (int j = i; j < DP; ++j) t = fma(v[j], q[f++], t);
-    s = fma(v[i], t, s);
-  }
+  for (int i = 0; i < DP; ++i)
+#pragma unroll
+    for (int j = i; j < DP; ++j) s = fma(v[i] * v[j], q[f++], s);
   return s;
 }
-
-__device__ __forceinline__ double linear_predict(const double* xr, const double* q, int d, int vec) {
-  double s = q[0];
+// `last`: the constant is the last feature (affine models), else the first
+__device__ __forceinline__ double linear_predict(const double* xr, const double* q, int d, int vec, bool last) {
+  double s = last ? 0.0 : q[0];
 #pragma unroll 4
   for (int i = 0; i < d; i += 8) {
     double v[8];
     load8(xr, i, d, vec, v);
 #pragma unroll
     for (int u = 0; u < 8; ++u) s = fma(v[u], q[1 + i + u], s);
+  }
+  return last ? s + q[0] : s;
+}
+// Feature by feature: with an infinite or NaN input the padding's products
+// (infinity times zero) must not enter.
+__device__ __noinline__ double plain_predict(const double* xr, const double* beta, int d, int kind, int p) {
+  double s = 0.0;
+  for (int f = 0; f < p; ++f) {
+    int a, b;
+    feature_factors(d, kind, f, a, b);
+    s = fma((a < 0 ? 1.0 : xr[a]) * (b < 0 ? 1.0 : xr[b]), beta[f], s);
   }
   return s;
 }
@@ -322,9 +334,10 @@ __global__ void __launch_bounds__(kLevelThreads)
       const double* xr = xk + r * d;
       const double yv = __ldg(y + r0 + r);
       double pred;
-      if (!quad) pred = linear_predict(xr, q, d, vec);
+      if (!quad) pred = linear_predict(xr, q, d, vec, kind == ART_FEATURES_AFFINE);
       else if (dp == 8) pred = quad_predict<8>(xr, q, d, vec);
       else pred = quad_predict<16>(xr, q, d, vec);
+      if (!isfinite(pred)) pred = plain_predict(xr, beta + k * bs, d, kind, p);
       const double e = yv - pred;
       s_e = fma(e, e, s_e);
       s_y = fma(yv, yv, s_y);
