@@ -9,9 +9,12 @@
 // |w . x - z|.
 #include <cooperative_groups.h>
 
-#include <utility>
+#include <algorithm>
+#include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
+#include "level_plan.cuh"
 #include "rows.cuh"
 
 namespace cg = cooperative_groups;
@@ -19,27 +22,80 @@ namespace cg = cooperative_groups;
 namespace art {
 namespace {
 
-// Both level kernels below give a node to a cluster of CTAs, since the nodes of
-// a level differ by a factor of a thousand in rows and one CTA reads only
-// about 50 GB/s.  The cluster's size follows the number of nodes (the more
-// nodes, the less a large one matters); what is added, and in which order,
-// follows the node's own row count, so results do not depend on it.
-// 307 nodes of 450 to 400,000 rows, d = 2 to 32 (1.7 GB): partition 14.5 ->
-// 0.59 ms, residuals 9.6 -> 0.65 ms against one CTA a node (2.6-2.9 TB/s of x
-// read once; before, the partition read it twice).
-constexpr int kLevelThreads = 256;
-constexpr int kLevelWarps = kLevelThreads / 32;
-constexpr int kMaxRanks = 16;  // CTAs of a cluster, and partial sums of a node, at most
+// The nodes of a level differ by a factor of a thousand in rows, and their sizes
+// are known on the device alone.  So a level call is two launches: the first deals
+// the nodes of at most `joint` rows to single CTAs (or, with several nodes a CTA,
+// those of at most `single` rows to its warps), the second each of the others to
+// a cluster of CTAs (one CTA reads about 50 GB/s).  The second starts as soon as
+// every CTA of the first has (programmatic dependent launch) and ends after it.
+// What is added, and in which order, follows the node's own row count, so results
+// depend on none of this.
+// A node of the level.
+struct LevelNode {
+  int64_t r0, n;
+  const double* x;
+  int d, vec;
+};
+__device__ __forceinline__ int64_t level_rows(const ArtSegments& seg, int64_t k) {
+  return seg.row_offsets[k + 1] - seg.row_offsets[k];
+}
+__device__ __forceinline__ LevelNode level_node(const ArtSegments& seg, const double* x, int64_t k) {
+  LevelNode v;
+  v.r0 = seg.row_offsets[k];
+  v.n = seg.row_offsets[k + 1] - v.r0;
+  v.x = x + seg.x_offsets[k];
+  v.d = seg.dims[k];
+  v.vec = row_vec(v.x, v.d);
+  return v;
+}
+// f with the width of a node's loads as a constant: a branch on it in every row
+// would keep the loads of several rows from being in flight together.
+template <typename F>
+__device__ __forceinline__ void by_width(int vec, F f) {
+  if (vec == 4) f(std::integral_constant<int, 4>());
+  else if (vec == 2) f(std::integral_constant<int, 2>());
+  else f(std::integral_constant<int, 1>());
+}
 
-int level_cluster(int64_t count) { return count <= 512 ? 16 : (count <= 2048 ? 8 : (count <= 8192 ? 4 : 1)); }
+// The first launch: single(node) by a warp, range(node) by the CTA.
+template <typename Range, typename Single>
+__device__ __forceinline__ void level_small_work(const ArtSegments& seg, const LevelPlan& L, Range range, Single single) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  const int64_t k0 = (int64_t)blockIdx.x * L.nodes;
+  const int nk = (int)min((int64_t)L.nodes, L.count - k0);
+  if (L.single >= 0)
+    for (int i = threadIdx.x >> 5; i < nk; i += kLevelWarps)
+      if (level_rows(seg, k0 + i) <= L.single) single(k0 + i);
+  for (int i = 0; i < nk; ++i) {
+    const int64_t n = level_rows(seg, k0 + i);
+    if (n > L.single && n <= L.joint) range(k0 + i);
+  }
+}
+// The second: range(node, how many before it) by the cluster; `hold`: what that
+// leaves in shared memory stays until every CTA has read it.
+template <bool hold, typename Range>
+__device__ __forceinline__ void level_large_work(const ArtSegments& seg, const LevelPlan& L, Range range) {
+  __shared__ unsigned big[kLevelWarps];
+  const int64_t k0 = (int64_t)(blockIdx.x / cg::this_cluster().num_blocks()) * L.nodes;
+  const int nk = (int)min((int64_t)L.nodes, L.count - k0), tid = threadIdx.x;
+  const unsigned m = __ballot_sync(0xffffffffu, tid < nk && level_rows(seg, k0 + tid) > L.joint);
+  if ((tid & 31) == 0) big[tid >> 5] = m;
+  if (__syncthreads_or(m != 0u)) {
+    int turn = 0;
+    for (int w = 0; 32 * w < nk; ++w)
+      for (unsigned left = big[w]; left; left &= left - 1u) range(k0 + 32 * w + __ffs(left) - 1, turn++);
+    if (hold) cg::this_cluster().sync();
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
-// right_side, decided by the plain score where that is further from zero
+// The side (right_side) is decided by the plain score where that is further from zero
 // than its error bound (gamma_{d+1} times sum |x_i w_i| + |z|, taken twice);
 // w is zero-padded to a multiple of eight.  Two FMAs an input against eleven
 // operations for the compensated score, which still decides the rest, NaN
 // and infinite scores and products near underflow among them.
-__device__ __forceinline__ bool row_side(const double* xr, const double* w, int d, double z, int vec) {
-  double s = 0.0, mag = 0.0;
+__device__ __forceinline__ void plain_score(const double* xr, const double* w, int d, int vec, double& s, double& mag) {
+  s = mag = 0.0;
 #pragma unroll 4
   for (int i = 0; i < d; i += 8) {
     double v[8];
@@ -50,12 +106,25 @@ __device__ __forceinline__ bool row_side(const double* xr, const double* w, int 
       mag = fma(fabs(v[q]), fabs(w[i + q]), mag);
     }
   }
+}
+__device__ __forceinline__ bool row_side(const double* xr, const double* w, int d, double z, int vec) {
+  double s, mag;
+  plain_score(xr, w, d, vec, s, mag);
   s = __dsub_rn(s, z);
   mag = __dadd_rn(mag, fabs(z));
-  const double bound = 2.220446049250313e-16 * (d + 4) * mag;
-  if (fabs(s) > bound && mag > 1e-280) return s >= 0.0;
+  if (fabs(s) > 2.220446049250313e-16 * (d + 4) * mag && mag > 1e-280) return s >= 0.0;
   return right_side(xr, w, d, z);
 }
+
+struct PartArgs {
+  ArtSegments seg;
+  const double* x;
+  const double* theta;
+  int64_t ts;
+  const int8_t* split;
+  int64_t* perm;
+  int32_t* n_right;
+};
 
 // Stable partition.  CTA r of a node's cluster takes the r-th range of its
 // rows: it reads x once, keeps the sides as a bit mask in shared memory, learns
@@ -63,101 +132,151 @@ __device__ __forceinline__ bool row_side(const double* xr, const double* w, int 
 // scatters its row numbers to their places.  Rows past the mask's capacity
 // (2^18 a CTA) have their sides formed a second time.
 constexpr int kMaskWords = 8192;
-__global__ void __launch_bounds__(kLevelThreads)
-    partition_kernel(ArtSegments seg, const double* x, const double* theta, int64_t ts,
-                     const int8_t* split, int64_t* perm, int32_t* n_right) {
+struct PartShared {
+  double w[kLevelWarps][ART_MAX_DIM + 8];  // zero-padded
+  int64_t right[2];
+  int warp[kLevelWarps];
+  unsigned mask[kMaskWords];
+};
+extern __shared__ __align__(16) unsigned char level_smem[];
+
+// This warp's rows first, first + step, ... (lane 0's; below end) to mask words
+// at, at + wstep, ... of shared memory, as far as there are any; returns the
+// right rows' number.
+__device__ __forceinline__ int mark_sides(const LevelNode& v, const double* w, double z, int64_t first, int64_t step, int64_t end,
+                                          int at, int wstep) {
+  PartShared& S = *(PartShared*)level_smem;
+  const int lane = threadIdx.x & 31;
+  int count = 0;
+#pragma unroll 1
+  for (int64_t r = first + lane; r - lane < end; r += step, at += wstep) {
+    const bool right = r < end && row_side(v.x + r * v.d, w, v.d, z, v.vec);
+    const unsigned m = __ballot_sync(0xffffffffu, right);
+    if (lane == 0 && at < kMaskWords) S.mask[at] = m;
+    count += __popc(m);
+  }
+  return count;
+}
+
+// This warp's words q of up to 32, a row per lane, to their places: `mine` is
+// word `lane`, `pre` the right rows before it (from `first` on), left and right
+// the next places.
+__device__ __forceinline__ void place_words(unsigned mine, int pre, int q0, int words, int64_t first, int64_t end,
+                                            int64_t r0, int64_t left, int64_t right, int64_t* perm) {
+  const int lane = threadIdx.x & 31;
+  for (int q = 0; q < 32; ++q) {
+    const int wq = q0 + q;
+    if (wq >= words) break;
+    const unsigned m = __shfl_sync(0xffffffffu, mine, q);
+    const int before = __shfl_sync(0xffffffffu, pre, q);
+    const int64_t r = first + 32 * (int64_t)wq + lane;
+    if (r < end) {
+      const int ahead = before + __popc(m & ((1u << lane) - 1u));
+      const int64_t pos = (m >> lane) & 1u ? right + ahead : left + (32 * wq + lane - ahead);
+      perm[r0 + pos] = r0 + r;
+    }
+  }
+}
+__device__ __forceinline__ int warp_scan(int v) {  // inclusive
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += t;
+  }
+  return v;
+}
+
+// One warp's node of at most kSingleRows rows.
+__device__ __forceinline__ void partition_warp(const PartArgs& A, int64_t k) {
+  PartShared& S = *(PartShared*)level_smem;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const LevelNode v = level_node(A.seg, A.x, k);
+  double* w = S.w[warp];
+  unsigned* mask = S.mask + 32 * warp;
+  __syncwarp();
+  for (int i = lane; i < ((v.d + 7) & ~7); i += 32) w[i] = i < v.d ? A.theta[k * A.ts + i] : 0.0;
+  mask[lane] = 0u;
+  const double z = A.theta[k * A.ts + v.d];
+  __syncwarp();
+  const int n = (int)v.n;
+  if (A.split == nullptr || A.split[k] != 0) mark_sides(v, w, z, 0, 32, n, 32 * warp, 1);
+  __syncwarp();
+  const unsigned mine = 32 * lane < n ? mask[lane] : 0u;
+  const int cnt = __popc(mine), incl = warp_scan(cnt), total = __shfl_sync(0xffffffffu, incl, 31);
+  if (A.n_right && lane == 0) A.n_right[k] = total;
+  place_words(mine, incl - cnt, 0, (n + 31) / 32, 0, n, v.r0, 0, n - total, A.perm);
+}
+
+// A CTA's range of a node: all of it, or its part of the cluster's, whose nodes
+// alternate between two slots for their counts (`turn`).
+template <bool CLUSTER>
+__device__ __forceinline__ void partition_range(const PartArgs& A, int64_t k, int turn) {
   cg::cluster_group cluster = cg::this_cluster();
-  const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-  const int64_t k = blockIdx.x / csize;
-  const int64_t r0 = seg.row_offsets[k], n = seg.row_offsets[k + 1] - r0;
-  const int64_t xoff = seg.x_offsets[k];
-  const int d = seg.dims[k];
-  const bool do_split = split == nullptr || split[k] != 0;
-  extern __shared__ unsigned mask[];
-  __shared__ double w[ART_MAX_DIM + 8];
-  __shared__ int64_t s_right;
-  __shared__ int s_warp[kLevelWarps];
-  __shared__ int pre[kLevelThreads];
+  const int csize = CLUSTER ? (int)cluster.num_blocks() : 1, crank = CLUSTER ? (int)cluster.block_rank() : 0;
+  PartShared& S = *(PartShared*)level_smem;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < ART_MAX_DIM + 8; i += kLevelThreads) w[i] = i < d ? theta[k * ts + i] : 0.0;
-  const double z = theta[k * ts + d];
-  const double* xk = x + xoff;
-  const int vec = row_vec(xk, d);
+  const LevelNode v = level_node(A.seg, A.x, k);
+  const int64_t n = v.n;
+  const bool do_split = A.split == nullptr || A.split[k] != 0;
+  double* w = S.w[0];
+  __syncthreads();  // the node before is done with what is shared
+  for (int i = tid; i < ((v.d + 7) & ~7); i += kLevelThreads) w[i] = i < v.d ? A.theta[k * A.ts + i] : 0.0;
+  const double z = A.theta[k * A.ts + v.d];
   const int64_t span = ((n + csize - 1) / csize + kLevelThreads - 1) / kLevelThreads * kLevelThreads;
   const int64_t a = min(n, span * crank), b = min(n, a + span);  // this CTA's rows
   __syncthreads();
-  int local = 0;
-#pragma unroll 2
-  for (int64_t base = a; base < b; base += kLevelThreads) {
-    const int64_t r = base + tid;
-    const bool right = do_split && r < b && row_side(xk + r * d, w, d, z, vec);
-    const unsigned m = __ballot_sync(0xffffffffu, right);
-    const int64_t word = (base - a) / 32 + warp;
-    if (lane == 0) {
-      local += __popc(m);
-      if (word < kMaskWords) mask[word] = m;
+  const int local = do_split ? mark_sides(v, w, z, a + 32 * warp, kLevelThreads, b, warp, kLevelWarps) : 0;
+  if (lane == 0) S.warp[warp] = local;
+  __syncthreads();
+  int64_t sum = 0;
+  for (int i = 0; i < kLevelWarps; ++i) sum += S.warp[i];
+  int64_t before = 0, total = sum;  // right rows of the ranges before this one, and of all
+  if (CLUSTER) {
+    if (tid == 0) S.right[turn & 1] = sum;
+    cluster.sync();
+    total = 0;
+    for (int c = 0; c < csize; ++c) {
+      const int64_t t = *cluster.map_shared_rank(&S.right[turn & 1], c);
+      if (c < crank) before += t;
+      total += t;
     }
   }
-  if (lane == 0) s_warp[warp] = local;
-  __syncthreads();
-  if (tid == 0) {
-    int64_t t = 0;
-    for (int i = 0; i < kLevelWarps; ++i) t += s_warp[i];
-    s_right = t;
-  }
-  cluster.sync();
-  int64_t before = 0, total = 0;  // right rows of the ranges before this one, and of all
-  for (int c = 0; c < csize; ++c) {
-    const int64_t v = *cluster.map_shared_rank(&s_right, c);
-    if (c < crank) before += v;
-    total += v;
-  }
-  if (n_right && crank == 0 && tid == 0) n_right[k] = (int32_t)total;
+  if (A.n_right && crank == 0 && tid == 0) A.n_right[k] = (int32_t)total;
   int64_t left = a - before, rgt = n - total + before;  // next places of this range
   for (int64_t base = a; base < b; base += 32 * kLevelThreads) {
     const int64_t words = min((int64_t)kLevelThreads, (b - base + 31) / 32);
     // exclusive prefix of the right counts of up to 256 words
     auto word_at = [&](int64_t q, int64_t row) -> unsigned {
       const int64_t at = (base - a) / 32 + q;
-      if (at < kMaskWords) return mask[at];
+      if (!do_split) return 0u;
+      if (at < kMaskWords) return S.mask[at];
       unsigned m = 0;
       for (int j = 0; j < 32 && row + j < b; ++j)
-        if (do_split && row_side(xk + (row + j) * d, w, d, z, vec)) m |= 1u << j;
+        if (row_side(v.x + (row + j) * v.d, w, v.d, z, v.vec)) m |= 1u << j;
       return m;
     };
     const unsigned mine = tid < words ? word_at(tid, base + 32 * tid) : 0u;
-    const int cnt = __popc(mine);
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
+    const int cnt = __popc(mine), incl = warp_scan(cnt);
     __syncthreads();
-    if (lane == 31) s_warp[warp] = incl;
+    if (lane == 31) S.warp[warp] = incl;
     __syncthreads();
     int wbase = 0, all = 0;
     for (int i = 0; i < kLevelWarps; ++i) {
-      if (i < warp) wbase += s_warp[i];
-      all += s_warp[i];
+      if (i < warp) wbase += S.warp[i];
+      all += S.warp[i];
     }
-    pre[tid] = wbase + incl - cnt;
-    __syncwarp();
-    for (int q = 0; q < 32; ++q) {  // this warp's 32 words, a row per lane
-      const int wq = 32 * warp + q;
-      if (wq >= words) break;
-      const unsigned m = __shfl_sync(0xffffffffu, mine, q);
-      const int64_t r = base + 32 * (int64_t)wq + lane;
-      if (r < b) {
-        const int ahead = pre[wq] + __popc(m & ((1u << lane) - 1u));
-        const int64_t pos = (m >> lane) & 1u ? rgt + ahead : left + (32 * wq + lane - ahead);
-        perm[r0 + pos] = r0 + r;
-      }
-    }
+    place_words(mine, wbase + incl - cnt, 32 * warp, (int)words, base, b, v.r0, left, rgt, A.perm);
     rgt += all;
     left += min((int64_t)32 * kLevelThreads, b - base) - all;
   }
-  cluster.sync();  // the counts stay until every CTA has read them
+}
+
+__global__ void __launch_bounds__(kLevelThreads, 4) partition_small(const __grid_constant__ PartArgs A, const LevelPlan L) {
+  level_small_work(A.seg, L, [&](int64_t k) { partition_range<false>(A, k, 0); }, [&](int64_t k) { partition_warp(A, k); });
+}
+__global__ void __launch_bounds__(kLevelThreads, 4) partition_large(const __grid_constant__ PartArgs A, const LevelPlan L) {
+  level_large_work<true>(A.seg, L, [&](int64_t k, int turn) { partition_range<true>(A, k, turn); });
 }
 
 // Tree walk and leaf prediction, a point per thread.  The nodes of a warp's
@@ -239,43 +358,132 @@ __global__ void __launch_bounds__(kPredictThreads)
 
 // Per segment: sum of squared residuals of phi(x) . beta and sum of y^2.  A
 // node's rows are cut into up to kMaxRanks ranges, fixed by its row count;
-// each range is one CTA's sum (threads in row order, then a fixed tree), and
-// the ranges are added in order.
+// each range is one CTA's sum (threads in row order, their sums added by warps
+// and the warps' in order), and the ranges are added in order.
 //
 // The features' products are formed and added in feature order, as
 // feature_factors gives it: the nested form x_i (b_i + sum b_ij x_j) has fewer
 // operations but other roundings, and overflows where the products do not.
-template <int DP>
-__device__ __forceinline__ double quad_predict(const double* xr, const double* q, int d, int vec) {
-  double v[DP];
-#pragma unroll
-  for (int i = 0; i < DP; i += 8) {
-    double t[8];
-    load8(xr, i, d, vec, t);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v[i + u] = t[u];
+struct ResArgs {
+  ArtSegments seg;
+  const double* x;
+  const double* y;
+  const double* beta;
+  int64_t bs;
+  double* sse;
+  double* ssy;
+};
+constexpr int kCoefs = ART_MAX_FEATURES + 24;  // by position: constant, a gap, inputs (zero-padded), products
+struct ResNode : LevelNode {
+  const double* beta;
+  const double* y;
+  const double* q;
+  int64_t span;
+  int kind, p, dp, ranks;  // dp: padded inputs of a quadratic model, else 0
+};
+struct ResShared {
+  double q[kLevelWarps][kCoefs];
+  double part[2][2][kMaxRanks];
+  double red[2][kMaxRanks][kLevelWarps];
+};
+
+// The coefficients of node k to q, by `threads` threads.
+template <int threads>
+__device__ __forceinline__ ResNode res_node(const ResArgs& A, int64_t k, double* q, int t) {
+  ResNode v;
+  (LevelNode&)v = level_node(A.seg, A.x, k);
+  v.kind = A.seg.features[k];
+  v.p = feature_count(v.d, v.kind);
+  v.beta = A.beta + k * A.bs;
+  v.y = A.y + v.r0;
+  v.q = q;
+  const bool quad = v.kind == ART_FEATURES_POLY2 || v.kind == ART_FEATURES_POLY2_NOBIAS;
+  v.dp = quad ? (v.d <= 8 ? 8 : 16) : 0;
+  v.ranks = (int)min((int64_t)kMaxRanks, (v.n + 1023) / 1024);
+  v.span = v.ranks ? (v.n + v.ranks - 1) / v.ranks : 0;
+  const int used = 2 + (quad ? v.dp + v.dp * (v.dp + 1) / 2 : v.d + 8);
+  auto sync = [] {
+    if (threads == 32) __syncwarp();
+    else __syncthreads();
+  };
+  sync();  // the node before is done with them
+  for (int i = t; i < used && i < kCoefs; i += threads) q[i] = 0.0;
+  sync();
+  for (int f = t; f < v.p; f += threads) {
+    int a, b;
+    feature_factors(v.d, v.kind, f, a, b);
+    int at;
+    if (a < 0) at = 0;
+    else if (b < 0) at = 2 + a;
+    else at = 2 + v.dp + a * v.dp - a * (a - 1) / 2 + (b - a);
+    if (at < kCoefs) q[at] = v.beta[f];
   }
-  double s = q[0];
-  int f = 1;
+  sync();
+  return v;
+}
+
+// A pair of coefficients, read where it is used: hoisted out of the row loop
+// they would fill the registers.
+__device__ __forceinline__ double2 coefs(const double* q) {
+  double2 c;
+  asm volatile("ld.volatile.shared.v2.f64 {%0, %1}, [%2];"
+               : "=d"(c.x), "=d"(c.y)
+               : "r"((uint32_t)__cvta_generic_to_shared(q)));
+  return c;
+}
+// Predictions of U rows, the rows' loads in flight together.
+template <int VEC, int DP, int U>
+__device__ __forceinline__ void quad_predict(const double* q, const double* const (&xr)[U], int d, double (&s)[U]) {
+  double v[U][DP];
 #pragma unroll
-  for (int i = 0; i < DP; ++i) s = fma(v[i], q[f++], s);
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int i = 0; i < DP; i += 8) load8(xr[u], i, d, VEC, *(double(*)[8]) & v[u][i]);
+  const double one = coefs(q).x;
+  double2 c;
+#pragma unroll
+  for (int u = 0; u < U; ++u) s[u] = one;
+#pragma unroll
+  for (int i = 0; i < DP; i += 2) {
+    c = coefs(q + 2 + i);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      s[u] = fma(v[u][i], c.x, s[u]);
+      s[u] = fma(v[u][i + 1], c.y, s[u]);
+    }
+  }
+  int f = 0;
 #pragma unroll
   for (int i = 0; i < DP; ++i)
 #pragma unroll
-    for (int j = i; j < DP; ++j) s = fma(v[i] * v[j], q[f++], s);
-  return s;
-}
-// `last`: the constant is the last feature (affine models), else the first
-__device__ __forceinline__ double linear_predict(const double* xr, const double* q, int d, int vec, bool last) {
-  double s = last ? 0.0 : q[0];
-#pragma unroll 4
-  for (int i = 0; i < d; i += 8) {
-    double v[8];
-    load8(xr, i, d, vec, v);
+    for (int j = i; j < DP; ++j, ++f) {
+      if ((f & 1) == 0) c = coefs(q + 2 + DP + f);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) s = fma(v[u], q[1 + i + u], s);
+      for (int u = 0; u < U; ++u) s[u] = fma(v[u][i] * v[u][j], f & 1 ? c.y : c.x, s[u]);
+    }
+}
+template <int VEC, int U>
+__device__ __forceinline__ void linear_predict(const double* q, const double* const (&xr)[U], int d, bool last, double (&s)[U]) {
+  const double one = coefs(q).x;  // the constant: an affine model's last feature, the others' first
+#pragma unroll
+  for (int u = 0; u < U; ++u) s[u] = last ? 0.0 : one;
+  for (int i = 0; i < d; i += 8) {
+    double v[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u) load8(xr[u], i, d, VEC, v[u]);
+#pragma unroll
+    for (int t = 0; t < 8; t += 2) {
+      const double2 c = coefs(q + 2 + i + t);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        s[u] = fma(v[u][t], c.x, s[u]);
+        s[u] = fma(v[u][t + 1], c.y, s[u]);
+      }
+    }
   }
-  return last ? s + q[0] : s;
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (last) s[u] += one;
 }
 // Feature by feature: with an infinite or NaN input the padding's products
 // (infinity times zero) must not enter.
@@ -288,107 +496,183 @@ __device__ __noinline__ double plain_predict(const double* xr, const double* bet
   }
   return s;
 }
+// The sums over rows first, first + kLevelThreads, ... below end, U rows at a
+// time; predict(rows, predictions).
+template <int U, typename F>
+__device__ __forceinline__ double2 res_loop(const double* x, const double* y, int d, int64_t first, int64_t end, bool& odd, F predict) {
+  double2 t = make_double2(0.0, 0.0);
+  for (int64_t r = first; r < end; r += U * kLevelThreads) {
+    const double* xr[U];
+    double yv[U], s[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t ru = r + u * kLevelThreads < end ? r + u * kLevelThreads : r;
+      xr[u] = x + ru * d;
+      yv[u] = __ldg(y + ru);
+    }
+    predict(xr, s);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (r + u * kLevelThreads < end) {
+        const double e = yv[u] - s[u];
+        odd |= !isfinite(s[u]);
+        t.x = fma(e, e, t.x);
+        t.y = fma(yv[u], yv[u], t.y);
+      }
+  }
+  return t;
+}
+__device__ __noinline__ double2 res_rows(const double* x, const double* y, const double* q, const double* beta, int d, int vec,
+                                         int dp, int kind, int p, int64_t first, int64_t end) {
+  bool odd = false;
+  double2 t;
+  by_width(vec, [&](auto v) {
+    if (dp == 0)
+      t = res_loop<2>(x, y, d, first, end, odd,
+                      [&](auto& xr, auto& s) { linear_predict<v>(q, xr, d, kind == ART_FEATURES_AFFINE, s); });
+    else if (dp == 8)
+      t = res_loop<2>(x, y, d, first, end, odd, [&](auto& xr, auto& s) { quad_predict<v, 8>(q, xr, d, s); });
+    else
+      t = res_loop<1>(x, y, d, first, end, odd, [&](auto& xr, auto& s) { quad_predict<v, 16>(q, xr, d, s); });
+  });
+  if (odd) {  // a prediction that is not finite: feature by feature
+    t.x = 0.0;
+    for (int64_t r = first; r < end; r += kLevelThreads) {
+      const double e = y[r] - plain_predict(x + r * d, beta, d, kind, p);
+      t.x = fma(e, e, t.x);
+    }
+  }
+  return t;
+}
 
-__global__ void __launch_bounds__(kLevelThreads)
-    residual_kernel(ArtSegments seg, const double* x, const double* y, const double* beta,
-                    int64_t bs, double* sse, double* ssy) {
+// One warp's node of one range: the CTA's order of additions.
+__device__ __forceinline__ void residual_warp(const ResArgs& A, int64_t k) {
+  ResShared& S = *(ResShared*)level_smem;
+  const int lane = threadIdx.x & 31;
+  const ResNode v = res_node<32>(A, k, S.q[threadIdx.x >> 5], lane);
+  double t_e = 0.0, t_y = 0.0;
+  for (int w = 0; 32 * w < v.n && w < kLevelWarps; ++w) {
+    const double2 t = res_rows(v.x, v.y, v.q, v.beta, v.d, v.vec, v.dp, v.kind, v.p, 32 * w + lane, v.n);
+    t_e += warp_sum(t.x);
+    t_y += warp_sum(t.y);
+  }
+  if (lane == 0) { A.sse[k] = t_e; A.ssy[k] = t_y; }
+}
+
+// A CTA's ranges of a node, all or every csize-th: their sums to the part array
+// of the cluster's CTA 0 (or its own), which adds them up.  The cluster's nodes
+// alternate between two arrays (`turn`).
+template <bool CLUSTER>
+__device__ __forceinline__ void residual_ranges(const ResArgs& A, int64_t k, int turn) {
   cg::cluster_group cluster = cg::this_cluster();
-  const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
-  // CTA 0 has started before its shared memory is written: waited for once the
-  // coefficients are in place
-  auto started = cluster.barrier_arrive();
-  const int64_t k = blockIdx.x / csize;
-  const int64_t r0 = seg.row_offsets[k], n = seg.row_offsets[k + 1] - r0;
-  const int64_t xoff = seg.x_offsets[k];
-  const int d = seg.dims[k], kind = seg.features[k];
-  const int p = feature_count(d, kind);
-  // coefficients by position: constant, inputs (zero-padded), products
-  __shared__ double q[ART_MAX_FEATURES + 8 + 16];
-  __shared__ double part[2][kMaxRanks];
-  __shared__ double red[2][kLevelWarps];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool quad = kind == ART_FEATURES_POLY2 || kind == ART_FEATURES_POLY2_NOBIAS;
-  const int dp = quad ? (d <= 8 ? 8 : 16) : d;
-  for (int i = tid; i < ART_MAX_FEATURES + 8 + 16; i += kLevelThreads) q[i] = 0.0;
-  __syncthreads();
-  for (int f = tid; f < p; f += kLevelThreads) {
-    int u, v;
-    feature_factors(d, kind, f, u, v);
-    int at;
-    if (u < 0) at = 0;
-    else if (v < 0) at = 1 + u;
-    else at = 1 + dp + u * dp - u * (u - 1) / 2 + (v - u);
-    if (at < ART_MAX_FEATURES + 24) q[at] = beta[k * bs + f];
+  const int csize = CLUSTER ? (int)cluster.num_blocks() : 1, crank = CLUSTER ? (int)cluster.block_rank() : 0;
+  ResShared& S = *(ResShared*)level_smem;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, slot = turn & 1;
+  const ResNode n = res_node<kLevelThreads>(A, k, S.q[0], tid);
+  if (CLUSTER && turn == 0) cluster.sync();  // CTA 0 has started before its shared memory is written
+  for (int v = crank; v < n.ranks; v += csize) {
+    const int64_t a = n.span * v, b = min(n.n, a + n.span);
+    const double2 t = res_rows(n.x, n.y, n.q, n.beta, n.d, n.vec, n.dp, n.kind, n.p, a + tid, b);
+    const double s_e = warp_sum(t.x), s_y = warp_sum(t.y);
+    if (lane == 0) { S.red[0][v][warp] = s_e; S.red[1][v][warp] = s_y; }
   }
   __syncthreads();
-  const double* xk = x + xoff;
-  const int vec = row_vec(xk, d);
-  const int ranks = (int)min((int64_t)kMaxRanks, (n + 1023) / 1024);
-  const int64_t span = ranks ? (n + ranks - 1) / ranks : 0;
-  cluster.barrier_wait(std::move(started));
-  for (int v = crank; v < ranks; v += csize) {
-    const int64_t a = span * v, b = min(n, a + span);
-    double s_e = 0.0, s_y = 0.0;
-#pragma unroll 2
-    for (int64_t r = a + tid; r < b; r += kLevelThreads) {
-      const double* xr = xk + r * d;
-      const double yv = __ldg(y + r0 + r);
-      double pred;
-      if (!quad) pred = linear_predict(xr, q, d, vec, kind == ART_FEATURES_AFFINE);
-      else if (dp == 8) pred = quad_predict<8>(xr, q, d, vec);
-      else pred = quad_predict<16>(xr, q, d, vec);
-      if (!isfinite(pred)) pred = plain_predict(xr, beta + k * bs, d, kind, p);
-      const double e = yv - pred;
-      s_e = fma(e, e, s_e);
-      s_y = fma(yv, yv, s_y);
-    }
-    s_e = warp_sum(s_e);
-    s_y = warp_sum(s_y);
-    if (lane == 0) { red[0][warp] = s_e; red[1][warp] = s_y; }
-    __syncthreads();
-    if (tid < 2) {
-      double t = 0.0;
-      for (int i = 0; i < kLevelWarps; ++i) t += red[tid][i];
-      *cluster.map_shared_rank(&part[tid][v], 0) = t;
-    }
-    __syncthreads();
+  const int v = tid >> 1, which = tid & 1;
+  if (v < n.ranks && v % csize == crank) {
+    double t = 0.0;
+    for (int i = 0; i < kLevelWarps; ++i) t += S.red[which][v][i];
+    double* at = &S.part[slot][which][v];
+    *(CLUSTER ? cluster.map_shared_rank(at, 0) : at) = t;
   }
-  cluster.sync();
+  if (CLUSTER) cluster.sync();
+  else __syncthreads();
   if (crank == 0 && tid < 2) {
     double t = 0.0;
-    for (int v = 0; v < ranks; ++v) t += part[tid][v];
-    (tid ? ssy : sse)[k] = t;
+    for (int i = 0; i < n.ranks; ++i) t += S.part[slot][tid][i];
+    (tid ? A.ssy : A.sse)[k] = t;
   }
 }
 
-template <typename... P, typename... A>
-int launch_level(void (*kern)(P...), int64_t count, size_t smem, cudaStream_t s, const char* what, A... args) {
-  const int c = level_cluster(count);
-  if ((c > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
-      (smem && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess))
-    return check_launch(what);
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)c;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)(count * c));
-  cfg.blockDim = dim3(kLevelThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  prof_begin(what, s);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
-  prof_end(s);
-  count_launch();
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    set_error("%s: %s", what, cudaGetErrorString(e));
-    return ART_E_LAUNCH;
-  }
-  return check_launch(what);
+__global__ void __launch_bounds__(kLevelThreads, 3) residual_small(const __grid_constant__ ResArgs A, const LevelPlan L) {
+  level_small_work(A.seg, L, [&](int64_t k) { residual_ranges<false>(A, k, 0); }, [&](int64_t k) { residual_warp(A, k); });
 }
+__global__ void __launch_bounds__(kLevelThreads, 3) residual_large(const __grid_constant__ ResArgs A, const LevelPlan L) {
+  level_large_work<false>(A.seg, L, [&](int64_t k, int turn) { residual_ranges<true>(A, k, turn); });
+}
+
+// A level's two kernels: attributes set, and the largest cluster of the second's
+// CTAs that fits the device (a fixed property) found, once per device.
+template <typename Args>
+struct LevelCall {
+  void (*small)(Args, LevelPlan);
+  void (*large)(Args, LevelPlan);
+  size_t smem;
+  std::atomic<int> cluster[64];
+
+  struct Config {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    Config(int64_t clusters, int c, size_t smem, bool after, cudaStream_t s) {
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)c;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.gridDim = dim3((unsigned)(clusters * c));
+      cfg.blockDim = dim3(kLevelThreads);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = s;
+      cfg.attrs = attr;
+      cfg.numAttrs = after ? 2 : 1;
+    }
+  };
+  int largest() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return 0; }
+    int c = cluster[dev].load(std::memory_order_acquire);
+    if (c > 0) return c;
+    for (auto kern : {small, large})
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+    cudaFuncSetAttribute(large, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    c = level_cluster([&](int size) {
+      const Config one(1, size, smem, false, nullptr);
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, large, &one.cfg) == cudaSuccess) return fit > 0;
+      cudaGetLastError();
+      return false;
+    });
+    cluster[dev].store(c, std::memory_order_release);
+    return c;
+  }
+  int run(int64_t count, cudaStream_t s, const char* what, const Args& args) {
+    const int c = largest();
+    if (c < 1) return check_launch(what);
+    const bool both = count > kLevelFew;
+    prof_begin(what, s);
+    cudaError_t e = cudaSuccess;
+    if (both) {
+      const LevelPlan L = level_small(count);
+      small<<<(unsigned)((count + L.nodes - 1) / L.nodes), kLevelThreads, smem, s>>>(args, L);
+      count_launch();
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
+      const LevelPlan L = level_large(count);
+      const Config config((count + L.nodes - 1) / L.nodes, c, smem, both, s);
+      e = cudaLaunchKernelEx(&config.cfg, large, args, L);
+      count_launch();
+    }
+    prof_end(s);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      set_error("%s: %s", what, cudaGetErrorString(e));
+      return ART_E_LAUNCH;
+    }
+    return check_launch(what);
+  }
+};
+LevelCall<ResArgs> g_residuals{residual_small, residual_large, sizeof(ResShared), {}};
+LevelCall<PartArgs> g_partition{partition_small, partition_large, sizeof(PartShared), {}};
 
 }  // namespace
 }  // namespace art
@@ -407,8 +691,8 @@ extern "C" int art_segment_residuals(const ArtSegments* seg, const double* x, co
     return ART_E_INVALID;
   }
   if (seg->count > 0x7fffffffll) { set_error("art_segment_residuals: too many segments"); return ART_E_UNSUPPORTED; }
-  return launch_level(residual_kernel, seg->count, 0, (cudaStream_t)stream, "segment_residuals", *seg, x, y, beta,
-                      beta_stride, sse, ssy);
+  return g_residuals.run(seg->count, (cudaStream_t)stream, "segment_residuals",
+                         ResArgs{*seg, x, y, beta, beta_stride, sse, ssy});
 }
 
 extern "C" int art_partition_rows(const ArtSegments* seg, const double* x, const double* theta,
@@ -419,8 +703,8 @@ extern "C" int art_partition_rows(const ArtSegments* seg, const double* x, const
   if (seg->count < 0 || seg->count > 0x7fffffff) { set_error("art_partition_rows: bad count"); return ART_E_INVALID; }
   if (seg->count == 0) return ART_OK;
   if (theta_stride < 2) { set_error("art_partition_rows: theta_stride too small"); return ART_E_INVALID; }
-  return launch_level(partition_kernel, seg->count, kMaskWords * sizeof(unsigned), (cudaStream_t)stream,
-                      "partition_rows", *seg, x, theta, theta_stride, split, perm, n_right);
+  return g_partition.run(seg->count, (cudaStream_t)stream, "partition_rows",
+                         PartArgs{*seg, x, theta, theta_stride, split, perm, n_right});
 }
 
 // Width of a table row's loads (see load8): whole sectors or pairs where every
