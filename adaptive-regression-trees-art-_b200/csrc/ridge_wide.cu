@@ -10,7 +10,8 @@
 // other is multiplied, with one block barrier a chunk; the row stride is 4
 // modulo 16 doubles, so that a fragment load (4 rows x 8 features) has no bank
 // conflicts.  Where the groups are fewer than the warps, several warps take a
-// group, each every other k-step, added in order at the end.
+// group, each every rg-th k-step of the system (whatever the chunks' length, which
+// follows the batch's widest system), added in order at the end.
 //
 // The finish factors the augmented system 8 columns at a time, the right-hand
 // side as one more row (so that only the back substitution is left), trailing
@@ -422,12 +423,13 @@ __global__ void __launch_bounds__(kWideThreads, 1) ridge_wide_kernel(RidgeArgs a
         // loops without a condition on any MMA: diagonal groups form their lower
         // blocks, the others all sixteen (columns past psi are zeros), or with
         // five group rows three block rows of four
-        const double* ph = buf + (4 * first + kq) * S + mq;
+        const int s0 = rg > 1 ? (int)((first + rg - (uint32_t)(ch % rg) * (CHUNK / 4) % rg) % rg) : 0;
+        const double* ph = buf + (4 * s0 + kq) * S + mq;
         const double *pi = ph + 32 * gi, *pj = ph + 32 * gj;
         const int step = 4 * rg * S;
         auto loop = [&](auto f) {
 #pragma unroll 2
-          for (int k0 = 4 * first; k0 < rows4; k0 += 4 * rg) {
+          for (int k0 = 4 * s0; k0 < rows4; k0 += 4 * rg) {
             f();
             ph += step;
             pi += step;
