@@ -236,6 +236,8 @@ def tune_ridge_threshold(x, y, w, row_offsets, dims, kinds, ridge, *, x_offsets=
 
 WARP_MAX_DIM = 23       # warp-per-restart form: inputs, features and trial steps it takes
 WARP_MAX_FEATURES = 23
+WARP_WIDE_DIM = 46      # ... with at most two restarts
+WARP_WIDE_FEATURES = 47
 WARP_MAX_TRIALS = 8
 
 

@@ -35,7 +35,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from . import _native as N
-from .autotune import WARP_MAX_DIM, WARP_MAX_FEATURES
+from .autotune import WARP_MAX_DIM, WARP_MAX_FEATURES, WARP_WIDE_DIM, WARP_WIDE_FEATURES
 
 WARP_MAX_ROWS = 1 << 16  # split nodes up to this size share the narrow launch
 from ._device import ptr, require_cuda, stream_handle, torch
@@ -85,6 +85,19 @@ class SurrogateJob:
     def n_final(self) -> int:
         per_round = int(round(self.grow_fraction * self.n_initial))
         return self.n_initial + self.rounds * per_round
+
+
+def _split_form(job: SurrogateJob, rows: int) -> tuple[int, ...]:
+    """Which split launch a node goes to: (0,) the narrow warp form's, which keeps
+    more warps on an SM; (1,) the wide warp form's (a node's split is the same in
+    either); wider models one launch per shape, since the CTA form's summation
+    order follows the launch's widest node."""
+
+    if job.dim <= WARP_MAX_DIM and job.n_features <= WARP_MAX_FEATURES and rows <= WARP_MAX_ROWS:
+        return (0,)
+    if job.dim <= WARP_WIDE_DIM and job.n_features <= WARP_WIDE_FEATURES:
+        return (1,)
+    return (2, job.dim, job.n_features)
 
 
 def job_footprint(job: SurrogateJob) -> int:
@@ -364,18 +377,15 @@ class ServingEngine:
                 split_idx.append(k)
         # max_iters is a per-call parameter of the split search (one call per
         # distinct value); the minimum side count goes per node, so nodes of
-        # every dimension share a launch.  Narrow nodes (d and p at most 23, at
-        # most WARP_MAX_ROWS rows) and the others go to separate launches: a
-        # launch's kernel follows its widest node, and the narrow one keeps more
-        # warps on an SM.  A node's split is the same in either.
-        groups: dict[tuple[int, bool], list[int]] = {}
+        # every dimension share a launch, as far as the form of the search allows
+        # (_split_form): a launch's form follows its widest node, and a node's
+        # split must not depend on the nodes batched with it.
+        groups: dict[tuple, list[int]] = {}
         for k in split_idx:
             job = work[k][0].job
-            warp = (job.dim <= WARP_MAX_DIM and job.n_features <= WARP_MAX_FEATURES
-                    and ro[k + 1] - ro[k] <= WARP_MAX_ROWS)
-            groups.setdefault((job.max_iters, warp), []).append(k)
-        for (iters, warp), ks in sorted(groups.items()):
-            self._split([work[k] for k in ks], x, y, ro, xo, d, kinds, ks, iters, warp)
+            groups.setdefault((job.max_iters, _split_form(job, int(ro[k + 1] - ro[k]))), []).append(k)
+        for (iters, form), ks in sorted(groups.items()):
+            self._split([work[k] for k in ks], x, y, ro, xo, d, kinds, ks, iters, form == (0,))
 
     def _split(self, sub, x, y, ro, xo, d, kinds, idx, iters, warp) -> None:
         t = torch()
