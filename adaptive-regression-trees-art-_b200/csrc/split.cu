@@ -1236,8 +1236,8 @@ __device__ void SplitCta<TC, TCG>::run(int item_id, int rank, int members) {
     }
     __syncthreads();
     // ---------------------------------------------------- line search
-    const int max_batches = (P.max_backtracks + 1 + a.H - 1) / a.H * P.max_line_search_failures + 1;
-    for (int batch = 0; batch < max_batches; ++batch) {
+    const int64_t max_batches = ((int64_t)P.max_backtracks + a.H) / a.H * P.max_line_search_failures + 1;
+    for (int64_t batch = 0; batch < max_batches; ++batch) {
       int any = 0;
       if (tid < it.rn) any = S(tid, RS_SEARCH) != 0.0;
       if (!__syncthreads_or(any)) break;
@@ -1267,7 +1267,7 @@ __device__ void SplitCta<TC, TCG>::run(int item_id, int rank, int members) {
         const int base = (int)S(r, RS_NBBASE);
         const double f0 = S(r, RS_LOSS), dd = S(r, RS_DD);
         int acc_j = -1;
-        for (int j = 0; j < H && base + j <= P.max_backtracks; ++j) {
+        for (int j = 0; j < H && j <= P.max_backtracks - base; ++j) {
           const double al = trial[r * H + j];
           const double rhs = __dadd_rn(f0, __dmul_rn(__dmul_rn(P.armijo_c, al), dd));
           if (trial[2 * a.Rg * H + r * H + j] <= rhs) { acc_j = j; break; }
@@ -1281,9 +1281,11 @@ __device__ void SplitCta<TC, TCG>::run(int item_id, int rank, int members) {
           step = trial[r * H + acc_j];
           nb = base + acc_j;
           S(r, RS_LSVAL) = trial[2 * a.Rg * H + r * H + acc_j];
-        } else if (base + H > P.max_backtracks) {
+        } else if (H > P.max_backtracks - base || trial[r * H + H - 1] == 0.0) {
+          // (a step that has underflowed to zero stays there: those after it are
+          // as unacceptable)
           attempt_done = true;
-          const int last = P.max_backtracks - base;
+          const int last = min(H - 1, P.max_backtracks - base);
           step = trial[r * H + last];
           nb = P.max_backtracks;
         } else {
@@ -1900,8 +1902,8 @@ extern "C" int art_split_level(const ArtSplitProblem* pr, const ArtSplitParams* 
     if (prm->precision == ART_PRECISION_MIXED && prm->tensor_gram && E <= kTcEntries) {
       int tc_cols = 2;
       const int rg = choose_rg(R, pa, prm->group_restarts, tc_cols);
-      const int H = std::min(std::min(prm->trial_steps > 0 ? prm->trial_steps : 4, std::max(1, kSplitThreads / std::max(rg, 1))),
-                             prm->max_backtracks + 1);
+      const int H = std::min(std::min(prm->trial_steps > 0 ? prm->trial_steps : 4, std::max(1, kSplitThreads / std::max(rg, 1))) - 1,
+                             prm->max_backtracks) + 1;
       if (rg >= 1 && split_layout(pr->max_dim, pr->max_features, rg, H, 2, kTcRows, 1).total <= 227 * 1024) {
         use_tc = 1;
         Rg = rg;
@@ -1938,7 +1940,7 @@ extern "C" int art_split_level(const ArtSplitProblem* pr, const ArtSplitParams* 
   // further passes), spare threads share the rows instead
   a.H = std::min(4, std::max(1, kSplitThreads / Rg));
   if (prm->trial_steps > 0) a.H = std::min(prm->trial_steps, std::max(1, kSplitThreads / Rg));
-  a.H = std::min(a.H, prm->max_backtracks + 1);
+  a.H = std::min(a.H - 1, prm->max_backtracks) + 1;
   a.r_theta = (double*)(ws + wl.r_theta); a.r_loss = (double*)(ws + wl.r_loss);
   a.r_beta = (double*)(ws + wl.r_beta); a.r_child = (double*)(ws + wl.r_child);
   a.r_ridge = (double*)(ws + wl.r_ridge);

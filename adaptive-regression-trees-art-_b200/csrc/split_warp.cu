@@ -1003,7 +1003,7 @@ __device__ __forceinline__ void SplitWarp<NB, SIDED>::run(int item) {
     double a_ = P.adaptive_alpha ? alpha : P.alpha0, step = 0.0;
     for (;;) {
       double al[kCand], f[kCand];
-      const int nc = min(kCand, P.max_backtracks - nb_ + 1);
+      const int nc = min(kCand - 1, P.max_backtracks - nb_) + 1;
       al[0] = a_;
 #pragma unroll
       for (int c = 1; c < kCand; ++c) al[c] = al[c - 1] * P.rho;
@@ -1030,15 +1030,17 @@ __device__ __forceinline__ void SplitWarp<NB, SIDED>::run(int item) {
         }
         break;
       }
-      nb_ += nc;
       double last = al[0];
 #pragma unroll
       for (int c = 1; c < kCand; ++c)
         if (c < nc) last = al[c];
-      if (nb_ <= P.max_backtracks) {  // next backtracks
+      if (P.max_backtracks - nb_ >= nc && last != 0.0) {  // next backtracks
+        nb_ += nc;
         a_ = last * P.rho;
         continue;
       }
+      // (a step that has underflowed to zero stays there: those after it are as
+      // unacceptable)
       // attempt failed: the last step tried
       if (P.adaptive_alpha) alpha = fmin(fmax(last * P.rho, P.alpha_min), P.alpha_max);
       ++failures;
