@@ -74,10 +74,12 @@ def _leaf_kind(model) -> int:
 
 
 def _sector_rows(n: int, columns: int) -> np.ndarray:
-    """Zeros (n, columns) in rows of whole 32-byte sectors: the device walk reads
-    such tables four doubles at a time."""
+    """Zeros (n, columns) in rows of whole 32-byte sectors, or of 16-byte pairs,
+    which the device walk reads four or two doubles at a time, where that adds
+    at most a third to the table (it is copied in every call)."""
 
-    return np.zeros((n, -(-columns // 4) * 4))[:, :columns]
+    width = next((w for w in (-(-columns // 4) * 4, -(-columns // 2) * 2) if 3 * w <= 4 * columns), columns)
+    return np.zeros((n, width))[:, :columns]
 
 
 class RegressionTree:

@@ -286,8 +286,28 @@ __global__ void __launch_bounds__(kLevelThreads, 4) partition_large(const __grid
 // waits in shared memory, [input][thread], where the features can index it.
 // 100,003 points of d = 8, depth 9, quadratic leaves: 52 us with single loads
 // of tables and points from memory, 31 us now.
+// W: doubles a block of loads, 8, or 2 for points of one or two inputs (eight
+// places of which one is used cost 2 M points of d = 1 27 %).
 constexpr int kPredictThreads = 128;
 
+template <int W>
+__device__ __forceinline__ void load_block(const double* x, int i, int d, int vec, double (&v)[W]) {
+  if constexpr (W == 8) {
+    load8(x, i, d, vec, v);
+  } else {
+    static_assert(W == 2);
+    if (vec >= 2) {
+      const double2 t = __ldg((const double2*)(x + i));
+      v[0] = t.x;
+      v[1] = t.y;
+    } else {
+      v[0] = __ldg(x + i);
+      v[1] = i + 1 < d ? __ldg(x + i + 1) : 0.0;
+    }
+  }
+}
+
+template <int W>
 __global__ void __launch_bounds__(kPredictThreads)
     predict_kernel(int d, int64_t n_nodes, const int32_t* child, const double* theta, int64_t ts, int wvec,
                    const double* coef, int64_t cs, int cvec, const int32_t* features, int64_t n, const double* x,
@@ -298,11 +318,11 @@ __global__ void __launch_bounds__(kPredictThreads)
   const double* xr = x + i * d;
   double* mine = sx + threadIdx.x;  // input c at mine[c * kPredictThreads]
   const int vec = row_vec(x, d);
-  for (int c = 0; c < d; c += 8) {
-    double v[8];
-    load8(xr, c, d, vec, v);
+  for (int c = 0; c < d; c += W) {
+    double v[W];
+    load_block<W>(xr, c, d, vec, v);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < W; ++q)
       if (c + q < d) mine[(c + q) * kPredictThreads] = v[q];
   }
   int node = 0;
@@ -311,11 +331,11 @@ __global__ void __launch_bounds__(kPredictThreads)
     const double z = t[d];
     // right_side by the plain score where its error bound allows, as row_side
     double s = 0.0, mag = 0.0;
-    for (int c = 0; c < d; c += 8) {
-      double w[8];
-      load8(t, c, d, wvec, w);
+    for (int c = 0; c < d; c += W) {
+      double w[W];
+      load_block<W>(t, c, d, wvec, w);
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
+      for (int q = 0; q < W; ++q)
         if (c + q < d) {  // z and whatever follows may share the last load
           const double v = mine[(c + q) * kPredictThreads];
           s = fma(v, w[q], s);
@@ -335,11 +355,11 @@ __global__ void __launch_bounds__(kPredictThreads)
   // features in order (feature_factors): factors a and b, -1 for a constant 1
   int a = kind == ART_FEATURES_POLY1 || kind == ART_FEATURES_POLY2 ? -1 : 0, b = -1;
   double s = 0.0;
-  for (int f = 0; f < p; f += 8) {
-    double c[8];
-    load8(co, f, p, cvec, c);
+  for (int f = 0; f < p; f += W) {
+    double c[W];
+    load_block<W>(co, f, p, cvec, c);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < W; ++q)
       if (f + q < p) {
         const double v = (a < 0 ? 1.0 : mine[a * kPredictThreads]) * (b < 0 ? 1.0 : mine[b * kPredictThreads]);
         s = fma(v, c[q], s);
@@ -728,11 +748,12 @@ extern "C" int art_tree_predict(int32_t dim, int64_t n_nodes, const int32_t* chi
   if (n_points <= 0) return ART_OK;
   const unsigned grid = (unsigned)((n_points + kPredictThreads - 1) / kPredictThreads);
   const size_t smem = sizeof(double) * dim * kPredictThreads;
+  const auto kern = dim <= 2 ? predict_kernel<2> : predict_kernel<8>;
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(predict_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return check_launch("art_tree_predict");
   prof_begin("tree_predict", (cudaStream_t)stream);
-  predict_kernel<<<grid, kPredictThreads, smem, (cudaStream_t)stream>>>(
+  kern<<<grid, kPredictThreads, smem, (cudaStream_t)stream>>>(
       dim, n_nodes, child, theta, theta_stride, table_vec(theta, theta_stride, dim), coef, coef_stride,
       table_vec(coef, coef_stride, 1), features, n_points, x, leaf, pred);
   prof_end((cudaStream_t)stream);
