@@ -139,6 +139,7 @@ class ArtChains(C.Structure):
 # Every entry point of include/art_b200.h with its ctypes signature.
 SIGNATURES = {
     "art_ridge_workspace_size": (C.c_size_t, [I64, I32]),
+    "art_ridge_workspace_size_rows": (C.c_size_t, [I64, I32, I64]),
     "art_ridge_batched": (C.c_int, [C.POINTER(ArtRidgeProblem), C.POINTER(ArtRidgeResult), P, C.c_size_t, P]),
     "art_ridge_noalloc_scratch_bytes": (C.c_size_t, []),
     "art_ridge_batched_noalloc": (C.c_int, [C.POINTER(ArtRidgeProblem), C.POINTER(ArtRidgeResult), P]),

@@ -352,7 +352,7 @@ def solve_weighted_ridge_batched(
         ptr(out.beta), int(out.beta.shape[1]), ptr(out.ridge_effective), ptr(out.cond_estimate),
         ptr(out.status), ptr(out.info),
     )
-    nbytes = lib.art_ridge_workspace_size(K, int(max_features))
+    nbytes = lib.art_ridge_workspace_size_rows(K, int(max_features), int(y.numel()))
     ws = WORKSPACES.get(nbytes, stream)
     rc = lib.art_ridge_batched(C.byref(prob), C.byref(res), ptr(ws), ws.numel(), stream_handle(stream))
     N.check(rc, "art_ridge_batched")
@@ -505,7 +505,7 @@ def ridge_gram_batched(x, y, weights, row_offsets, dims, features, *, x_offsets=
     seg = N.ArtSegments(K, ptr(ro), ptr(xo), ptr(dims_t), ptr(feats))
     prob = N.ArtRidgeProblem(seg, ptr(x), ptr(y), ptr(w), ptr(ridge_t), float(weight_floor), N.SOLVER_NORMAL,
                              N.PRECISION_MIXED, 1e-10, int(max_features), int(max_dim), 0, 0)
-    nbytes = lib.art_ridge_workspace_size(K, int(max_features))
+    nbytes = lib.art_ridge_workspace_size_rows(K, int(max_features), 0)  # no system is split
     ws = WORKSPACES.get(nbytes, stream)
     rc = lib.art_ridge_gram(C.byref(prob), ptr(gram), E, ptr(status), ptr(ws), ws.numel(), stream_handle(stream))
     N.check(rc, "art_ridge_gram")

@@ -567,6 +567,16 @@ extern "C" size_t art_ridge_workspace_size(int64_t count, int32_t max_features) 
   return split_layout(count, std::max(max_features, 1), ws_layout(count).total).total;
 }
 
+extern "C" size_t art_ridge_workspace_size_rows(int64_t count, int32_t max_features, int64_t rows) {
+  if (count < 0) return 0;
+  const int p = std::max(max_features, 1);
+  const SplitLayout sl = split_layout(count, p, ws_layout(count).total);
+  if (sl.rec_cap == 0) return sl.total;
+  // a split system has at least two units, all but its last of 256 rows or more
+  const size_t pa = std::min(p, kSmallMaxAug - 1) + 1, units = (size_t)(std::max<int64_t>(rows, 0) / 128);
+  return std::min(sl.total, sl.off_pool + (units * (pa * (pa + 1) / 2) * sizeof(double) + 255) / 256 * 256);
+}
+
 static int ridge_entry(const ArtRidgeProblem* pr, const ArtRidgeResult* res, float* gram_out,
                        int64_t gram_stride, void* workspace, size_t ws_bytes, art_stream_t stream) {
   if (!pr || !res) { set_error("art_ridge_batched: null problem/result"); return ART_E_INVALID; }

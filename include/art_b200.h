@@ -159,6 +159,9 @@ typedef struct ArtRidgeResult {
  * 256 MiB) to split large systems over many warps; a call given less, down to
  * the lists alone, splits fewer of them, with the same results.              */
 ART_API size_t art_ridge_workspace_size(int64_t count, int32_t max_features);
+/* The part of it that a batch of at most `rows` rows in all can use: as many
+ * systems are split as with the whole.                                       */
+ART_API size_t art_ridge_workspace_size_rows(int64_t count, int32_t max_features, int64_t rows);
 /* Weighted Grams only, by the mixed form's tensor-core path: for every system
  * with 33 <= p <= 160 and d <= ART_MAX_DIM, G' = sum_k q_k phi_k phi_k^T from
  * TF32 hi/lo split products accumulated in FP32, written as the packed lower
