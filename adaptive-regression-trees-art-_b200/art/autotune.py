@@ -266,6 +266,19 @@ def split_candidates(R: int, max_backtracks: int, d: int = 0, p: int = 0,
     return out
 
 
+def _distinct_launches(candidates, R: int, d: int, p: int, tensor_gram: bool = False):
+    """One shape for each launch the library makes of them: with at most two restarts every shape
+    that fits the warp form runs it, and that form takes no trial steps."""
+
+    every = R <= 2 and d <= WARP_WIDE_DIM and p <= WARP_WIDE_FEATURES and not tensor_gram
+    seen = {}
+    for c in candidates:
+        key = "warp" if c[3] or every else c
+        if key not in seen or (c[3] and not seen[key][3]):
+            seen[key] = c
+    return list(seen.values())
+
+
 def tune_split_shape(splitter, x, y, row_offsets, dims, features, temperature, ridge, *, max_dim: int,
                      max_features: int, theta0=None, anneal_ratio: float = 1.0, hard_refit: bool = True,
                      repeats: int = 2, stream=None) -> dict:
@@ -278,7 +291,8 @@ def tune_split_shape(splitter, x, y, row_offsets, dims, features, temperature, r
     R = int(max(1, splitter.n_restarts))
     tc = bool(getattr(splitter, "tensor_gram", False)) and getattr(splitter, "precision", "fp64") == "mixed"
     timings = {}
-    for g, h, c, w in split_candidates(R, int(splitter.max_backtracks), int(max_dim), int(max_features), tc):
+    shapes = split_candidates(R, int(splitter.max_backtracks), int(max_dim), int(max_features), tc)
+    for g, h, c, w in _distinct_launches(shapes, R, int(max_dim), int(max_features), tc):
         def run(g=g, h=h, c=c, w=w):
             return split_level(splitter, x, y, row_offsets, dims, features, temperature, ridge, theta0=theta0,
                                anneal_ratio=anneal_ratio, hard_refit=hard_refit, max_dim=max_dim,
