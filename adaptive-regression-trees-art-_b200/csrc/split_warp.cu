@@ -919,7 +919,7 @@ __device__ __forceinline__ void SplitWarp<NB, SIDED>::run(int item) {
   // Affine models whose inputs fill whole blocks, at most one input a lane (and
   // side): 1 and y would take a block row of their own, of which two columns of
   // eight are used.  256 nodes of d = 16, 16 restarts: 71.6 ms to 69.9; 149 nodes
-  // to 120,000 rows, d = 32 or quadratic of d = 8: 24.9 ms to 23.9.
+  // to 120,000 rows, d = 32 or quadratic of d = 8: 24.9 ms to 24.2.
   apart = NB > 1 && NB <= 5 && kind == ART_FEATURES_AFFINE && tail <= 2;
 #pragma unroll
   for (int I = 0; I < NB; ++I) {

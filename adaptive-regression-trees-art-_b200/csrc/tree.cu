@@ -285,7 +285,8 @@ __global__ void __launch_bounds__(kLevelThreads, 4) partition_large(const __grid
 // sectors (wvec, cvec: see load8) are read four doubles at a time.  The point
 // waits in shared memory, [input][thread], where the features can index it.
 // 100,003 points of d = 8, depth 9, quadratic leaves: 52 us with single loads
-// of tables and points from memory, 31 us now.
+// of tables and points from memory, 31 us now; of d = 64, depth 10, affine leaves (64 KB
+// of points a CTA, three CTAs an SM): 386 and 114 us.
 // W: doubles a block of loads, 8, or 2 for points of one or two inputs (eight
 // places of which one is used cost 2 M points of d = 1 27 %).
 constexpr int kPredictThreads = 128;
