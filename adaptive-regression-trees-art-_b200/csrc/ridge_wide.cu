@@ -389,6 +389,9 @@ __global__ void __launch_bounds__(kWideThreads, 1) ridge_wide_kernel(RidgeArgs a
       g1 = g0 + F * 2;
       gs = 1;
     }
+    // this warp's first k-step in the chunk, so that it takes every rg-th of the system
+    int s0 = first;
+    const int back = (CHUNK / 4) % rg;
     for (int64_t ch = 0; ch < nchunks; ++ch) {
       const int st = (int)(ch & 1);
       const int rows = (int)min((int64_t)CHUNK, it.n - ch * CHUNK), rows4 = (rows + 3) & ~3;
@@ -423,7 +426,6 @@ __global__ void __launch_bounds__(kWideThreads, 1) ridge_wide_kernel(RidgeArgs a
         // loops without a condition on any MMA: diagonal groups form their lower
         // blocks, the others all sixteen (columns past psi are zeros), or with
         // five group rows three block rows of four
-        const int s0 = rg > 1 ? (int)((first + rg - (uint32_t)(ch % rg) * (CHUNK / 4) % rg) % rg) : 0;
         const double* ph = buf + (4 * s0 + kq) * S + mq;
         const double *pi = ph + 32 * gi, *pj = ph + 32 * gj;
         const int step = 4 * rg * S;
@@ -500,6 +502,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) ridge_wide_kernel(RidgeArgs a
           });
         }
       }
+      s0 -= back;
+      if (s0 < 0) s0 += rg;
       if (extra && tid < p)
         for (int r = 0; r < rows; ++r) hx = fma(buf[r * S + tid], buf[r * S + 8 * kMaxBlocks], hx);
     }
