@@ -27,11 +27,12 @@ struct LevelPlan {
 // 1,000 nodes of 450 to 20,000 rows: 0.30 ms at 8,192 to 10,240, 0.38 at 20,480).
 // 444 CTAs for the first launch (three an SM, all resident) until that is eight
 // nodes each, which their warps take side by side; 148 clusters for the second:
-// 296 cost levels of small nodes 2 to 4 us more, 74 the large ones 3 %.
+// 296 cost levels of small nodes 2 to 4 us more, 74 the large ones 3 %.  (`ctas`: the
+// first launch's where another kernel makes it.)
 constexpr int64_t kLevelFew = 32;
 inline int64_t level_joint(int64_t count) { return 2048 * std::min<int64_t>(std::max<int64_t>(count / 100, 1), 4); }
-inline LevelPlan level_small(int64_t count) {
-  LevelPlan L{count, level_joint(count), (int)std::min<int64_t>((count + 443) / 444, 8), -1};
+inline LevelPlan level_small(int64_t count, int ctas = 444) {
+  LevelPlan L{count, level_joint(count), (int)std::min<int64_t>((count + ctas - 1) / ctas, 8), -1};
   if (L.nodes > 1) L.single = std::min(kSingleRows, 128 * L.nodes);
   return L;
 }

@@ -614,6 +614,134 @@ __device__ __forceinline__ void residual_ranges(const ResArgs& A, int64_t k, int
   }
 }
 
+// The first launch for levels of up to kNarrowFeatures features (the stride of
+// beta says so): the general kernel pads a row to eight inputs and holds 80
+// registers, three CTAs an SM, and for such rows latency is most of its time.
+// Here a row takes its features one at a time; the order of additions, and so the
+// result, is the general kernel's.  Any node is right, only its time depends on
+// its features.  Five CTAs an SM and one node a CTA up to four times as many
+// (general kernel -> this one): d = 1, 600 nodes of 5,000 rows 37 -> 23 us, 3,000
+// of 2,000 70 -> 43, 12,000 of 600 89 -> 67; d = 5, 55 -> 44, 88 -> 80, 118 -> 117;
+// 3,000 of 64 rows 17 -> 19.  With eight features it loses (12,000 of 600: 141 us
+// and 190).  Six and eight CTAs an SM (40 and 32 registers) take 74 and 119 us for
+// 12,000 of 600, d = 1.
+constexpr int kNarrowFeatures = 6;
+constexpr int kNarrowCtas = 5;  // an SM
+constexpr int kNarrowGrid = 148 * kNarrowCtas * 4;
+struct NarrowShared {
+  double b[kLevelWarps][ART_MAX_FEATURES];
+  int16_t fa[kLevelWarps][ART_MAX_FEATURES], fb[kLevelWarps][ART_MAX_FEATURES];
+  double part[2][kMaxRanks];
+  double red[2][kMaxRanks][kLevelWarps];
+};
+// The node's coefficients and their factors, by `threads` threads; how many.
+template <int threads>
+__device__ __forceinline__ int narrow_node(const ResArgs& A, int64_t k, int d, NarrowShared& S, int at, int t) {
+  const int kind = A.seg.features[k], p = min(feature_count(d, kind), ART_MAX_FEATURES);
+  const double* beta = A.beta + k * A.bs;
+  if (threads == 32) __syncwarp();
+  else __syncthreads();
+  for (int f = t; f < p; f += threads) {
+    int a, b;
+    feature_factors(d, kind, f, a, b);
+    S.fa[at][f] = (int16_t)a;
+    S.fb[at][f] = (int16_t)b;
+    S.b[at][f] = beta[f];
+  }
+  if (threads == 32) __syncwarp();
+  else __syncthreads();
+  return p;
+}
+// Rows r, r + step, ... (U of them, below end): added to t[0], or each to its t[u].
+template <int U, int SUMS>
+__device__ __forceinline__ void narrow_rows(const NarrowShared& S, int at, int p, const double* x, const double* y, int d, int64_t r,
+                                            int step, int64_t end, double2 (&t)[SUMS]) {
+  const double* xr[U];
+  double yv[U], s[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t ru = r + u * step < end ? r + u * step : r;
+    xr[u] = x + ru * d;
+    yv[u] = __ldg(y + ru);
+    s[u] = 0.0;
+  }
+#pragma unroll 2
+  for (int f = 0; f < p; ++f) {
+    const int a = S.fa[at][f], b = S.fb[at][f];
+    const double c = S.b[at][f];
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = a < 0 ? 1.0 : __ldg(xr[u] + a);
+    if (b >= 0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] *= __ldg(xr[u] + b);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) s[u] = fma(v[u], c, s[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (r + u * step < end) {
+      double2& q = t[SUMS == 1 ? 0 : u];
+      const double e = yv[u] - s[u];
+      q.x = fma(e, e, q.x);
+      q.y = fma(yv[u], yv[u], q.y);
+    }
+}
+// residual_warp and residual_ranges<false>, feature by feature.
+__device__ __forceinline__ void narrow_warp(const ResArgs& A, int64_t k) {
+  NarrowShared& S = *(NarrowShared*)level_smem;
+  const int lane = threadIdx.x & 31, at = threadIdx.x >> 5;
+  const LevelNode v = level_node(A.seg, A.x, k);
+  const double* y = A.y + v.r0;
+  const int p = narrow_node<32>(A, k, v.d, S, at, lane);
+  double t_e = 0.0, t_y = 0.0;
+  constexpr int W = 4;  // of the CTA's warps side by side
+  for (int w = 0; 32 * w < v.n && w < kLevelWarps; w += W) {
+    double2 t[W];
+#pragma unroll
+    for (int u = 0; u < W; ++u) t[u] = make_double2(0.0, 0.0);
+    for (int64_t r = 32 * w + lane; r < v.n; r += kLevelThreads) narrow_rows<W, W>(S, at, p, v.x, y, v.d, r, 32, v.n, t);
+#pragma unroll
+    for (int u = 0; u < W; ++u) {
+      t_e += warp_sum(t[u].x);
+      t_y += warp_sum(t[u].y);
+    }
+  }
+  if (lane == 0) { A.sse[k] = t_e; A.ssy[k] = t_y; }
+}
+__device__ __forceinline__ void narrow_range(const ResArgs& A, int64_t k) {
+  NarrowShared& S = *(NarrowShared*)level_smem;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const LevelNode v = level_node(A.seg, A.x, k);
+  const double* y = A.y + v.r0;
+  const int p = narrow_node<kLevelThreads>(A, k, v.d, S, 0, tid);
+  const int ranks = (int)min((int64_t)kMaxRanks, (v.n + 1023) / 1024);
+  const int64_t span = ranks ? (v.n + ranks - 1) / ranks : 0;
+  for (int q = 0; q < ranks; ++q) {
+    const int64_t a = span * q, b = min(v.n, a + span);
+    double2 t[1] = {make_double2(0.0, 0.0)};
+    for (int64_t r = a + tid; r < b; r += 2 * kLevelThreads) narrow_rows<2, 1>(S, 0, p, v.x, y, v.d, r, kLevelThreads, b, t);
+    const double s_e = warp_sum(t[0].x), s_y = warp_sum(t[0].y);
+    if (lane == 0) { S.red[0][q][warp] = s_e; S.red[1][q][warp] = s_y; }
+  }
+  __syncthreads();
+  const int q = tid >> 1, which = tid & 1;
+  if (q < ranks) {
+    double t = 0.0;
+    for (int i = 0; i < kLevelWarps; ++i) t += S.red[which][q][i];
+    S.part[which][q] = t;
+  }
+  __syncthreads();
+  if (tid < 2) {
+    double t = 0.0;
+    for (int i = 0; i < ranks; ++i) t += S.part[tid][i];
+    (tid ? A.ssy : A.sse)[k] = t;
+  }
+}
+__global__ void __launch_bounds__(kLevelThreads, kNarrowCtas) residual_narrow(const __grid_constant__ ResArgs A, const LevelPlan L) {
+  level_small_work(A.seg, L, [&](int64_t k) { narrow_range(A, k); }, [&](int64_t k) { narrow_warp(A, k); });
+}
 __global__ void __launch_bounds__(kLevelThreads, 3) residual_small(const __grid_constant__ ResArgs A, const LevelPlan L) {
   level_small_work(A.seg, L, [&](int64_t k) { residual_ranges<false>(A, k, 0); }, [&](int64_t k) { residual_warp(A, k); });
 }
@@ -665,15 +793,15 @@ struct LevelCall {
     cluster[dev].store(c, std::memory_order_release);
     return c;
   }
-  int run(int64_t count, cudaStream_t s, const char* what, const Args& args) {
+  int run(int64_t count, cudaStream_t s, const char* what, const Args& args, void (*lean)(Args, LevelPlan) = nullptr) {
     const int c = largest();
     if (c < 1) return check_launch(what);
     const bool both = count > kLevelFew;
     prof_begin(what, s);
     cudaError_t e = cudaSuccess;
     if (both) {
-      const LevelPlan L = level_small(count);
-      small<<<(unsigned)((count + L.nodes - 1) / L.nodes), kLevelThreads, smem, s>>>(args, L);
+      const LevelPlan L = lean ? level_small(count, kNarrowGrid) : level_small(count);
+      (lean ? lean : small)<<<(unsigned)((count + L.nodes - 1) / L.nodes), kLevelThreads, lean ? sizeof(NarrowShared) : smem, s>>>(args, L);
       count_launch();
       e = cudaGetLastError();
     }
@@ -713,7 +841,7 @@ extern "C" int art_segment_residuals(const ArtSegments* seg, const double* x, co
   }
   if (seg->count > 0x7fffffffll) { set_error("art_segment_residuals: too many segments"); return ART_E_UNSUPPORTED; }
   return g_residuals.run(seg->count, (cudaStream_t)stream, "segment_residuals",
-                         ResArgs{*seg, x, y, beta, beta_stride, sse, ssy});
+                         ResArgs{*seg, x, y, beta, beta_stride, sse, ssy}, beta_stride <= kNarrowFeatures ? residual_narrow : nullptr);
 }
 
 extern "C" int art_partition_rows(const ArtSegments* seg, const double* x, const double* theta,
